@@ -278,8 +278,12 @@ struct pale_handle {
   int timed = 0;           // 1 forward events, 2 adjoint events pending
   cudaStream_t own_stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
+  cudaEvent_t round_ev = nullptr;     // behind a gather round's queue length
+  uint32_t* h_live = nullptr;         // pinned: that length
 
   ~pale_handle() {
+    if (round_ev) cudaEventDestroy(round_ev);
+    if (h_live) cudaFreeHost(h_live);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (ev2) cudaEventDestroy(ev2);
@@ -1003,6 +1007,8 @@ FrameArgs frame_args(const std::vector<pale_handle*>& scenes, uint32_t nsel, uin
   F.path_capacity = h->path_cap;
   F.walk_block = h->st.walk_block;
   F.timer = &h->timer;
+  F.h_live = h->h_live;
+  F.round_ev = h->round_ev;
   return F;
 }
 
@@ -1557,6 +1563,8 @@ int pale_create(const pale_scene_desc* desc, const pale_settings* settings, pale
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
     CK(cudaEventCreate(&h->ev2));
+    CK(cudaEventCreateWithFlags(&h->round_ev, cudaEventDisableTiming));
+    CK(cudaMallocHost(&h->h_live, 64));
     setup_scene(h, desc);
     return PALE_OK;
   });

@@ -263,6 +263,10 @@ struct FrameArgs {
   float4* walk;
   uint32_t* khit;
   KernelTimer* timer;      // host side, may be null
+  // host side: a pinned word the length of the next round's queue is copied
+  // to, and the event behind that copy
+  volatile uint32_t* h_live;
+  cudaEvent_t round_ev;
   // optional L2 image loss: target packed like the images with
   // target_channels floats per pixel; dL/dI (float4 per pixel) written by
   // the post-process

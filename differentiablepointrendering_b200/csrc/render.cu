@@ -1009,26 +1009,29 @@ uint32_t gather_rounds(const FrameArgs& a, const GatherShape& g, uint32_t n, cud
   cudaMemsetAsync(a.counts, 0, 2 * (kMaxLayers + 2) * sizeof(uint32_t), s);
   k_cg_init<<<blocks_for(n), kBlock, 0, s>>>(a, n); note_launch();
   // every round consumes at least one layer of each live path, so
-  // kMaxLayers rounds bound the walk (the layer cap ends longer ones)
+  // kMaxLayers rounds bound the walk (the layer cap ends longer ones).
+  // The length of the next round's queue is known once k_cg_round has run:
+  // its copy to the host is queued behind that kernel, the round's lookups
+  // behind the copy, and the host waits for the copy only, so that it
+  // queues the next round (or ends) while the lookups run.
   uint32_t round = 0, live = n;
   while (round < (uint32_t)kMaxLayers && live) {
-    for (uint32_t group = 0; group < 16 && round < (uint32_t)kMaxLayers; ++group, ++round) {
-      if (a.timer) a.timer->begin(kTimeTrace, s);
-      k_cg_mesh<<<g.grid_r, kBlock, 0, s>>>(a, round); note_launch();
-      if (g.wt == 64) launch_walk(k_cg_walk<kGatherHits, kMulti, 64>, 64, a, round, g.smem, ~0u, s);
-      else if (g.wt == 128) launch_walk(k_cg_walk<kGatherHits, kMulti, 128>, 128, a, round, g.smem, ~0u, s);
-      else launch_walk(k_cg_walk<kGatherHits, kMulti, 256>, 256, a, round, g.smem, ~0u, s);
-      k_cg_round<kGatherHits><<<g.grid_r, kBlock, 0, s>>>(a, round); note_launch();
-      if (a.timer) a.timer->end(s);
-      if (a.timer) a.timer->begin(kTimeLookup, s);
-      k_cg_lookup<kMulti><<<g.grid_l, kBlock, 0, s>>>(a, round); note_launch();
-      if (a.timer) a.timer->end(s);
-      // queues only shrink, so `live` bounds the entries of every round of the group
-      k_cg_compose<<<blocks_for(live), kBlock, 0, s>>>(a, round); note_launch();
-    }
-    // the host reads the queue length after each group of 16 rounds
-    cudaMemcpyAsync(&live, a.counts + round, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    cudaStreamSynchronize(s);
+    if (a.timer) a.timer->begin(kTimeTrace, s);
+    k_cg_mesh<<<g.grid_r, kBlock, 0, s>>>(a, round); note_launch();
+    if (g.wt == 64) launch_walk(k_cg_walk<kGatherHits, kMulti, 64>, 64, a, round, g.smem, ~0u, s);
+    else if (g.wt == 128) launch_walk(k_cg_walk<kGatherHits, kMulti, 128>, 128, a, round, g.smem, ~0u, s);
+    else launch_walk(k_cg_walk<kGatherHits, kMulti, 256>, 256, a, round, g.smem, ~0u, s);
+    k_cg_round<kGatherHits><<<g.grid_r, kBlock, 0, s>>>(a, round); note_launch();
+    if (a.timer) a.timer->end(s);
+    cudaMemcpyAsync(const_cast<uint32_t*>(a.h_live), a.counts + round + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
+    cudaEventRecord(a.round_ev, s);
+    if (a.timer) a.timer->begin(kTimeLookup, s);
+    k_cg_lookup<kMulti><<<g.grid_l, kBlock, 0, s>>>(a, round); note_launch();
+    if (a.timer) a.timer->end(s);
+    k_cg_compose<<<blocks_for(live), kBlock, 0, s>>>(a, round); note_launch();
+    ++round;
+    if (cudaEventSynchronize(a.round_ev) != cudaSuccess) break;   // the caller reports the error
+    live = *a.h_live;
   }
   return round;
 }
