@@ -213,7 +213,7 @@ struct pale_handle {
   DBuf<float4> ph_a, ph_b, ph_sa, ph_sb, g_pa, g_pb;
   DBuf<float> ph_c, ph_sc, g_pc;
   DBuf<uint32_t> g_cell_id, g_sorted, g_keys, g_vals_tmp, g_sort_temp, g_cell_count, g_cell_off, g_scan_temp,
-      g_stored, g_attempts;
+      g_stored, g_attempts, g_lit, g_lit_x;
   // queues
   uint32_t qcap = 0;
   DBuf<RayRec> q0, q1, qstage;
@@ -236,8 +236,11 @@ struct pale_handle {
   DBuf<RayRec> cg_paths, cg_paths2;
   DBuf<float4> cg_qrec, cg_info_b;
   DBuf<uint4> cg_info_a;
-  DBuf<float4> cg_mhit, cg_walk;   // per round entry: mesh hit, walk record
-  DBuf<uint32_t> cg_khit;          // per round entry: K-hit walk result
+  // per round entry the mesh hit (1 float4), the walk record (2) and the
+  // K-hit walk result (kKHitWords words); then, in the same memory, the
+  // round's lookups (per record 2 words, then 1)
+  DBuf<float4> cg_entry;
+  DBuf<uint32_t> cg_bins;
   DBuf<uint32_t> cg_counts;
   DBuf<float4> cg_res, cg_fb;
   // run state, seeds, images, gradients
@@ -324,6 +327,8 @@ struct pale_handle {
     g.pa = g_pa.p;
     g.pb = g_pb.p;
     g.pc = g_pc.p;
+    g.lit = g_lit.p;
+    g.lit_row = ((uint32_t)res[0] + 31u) / 32u;
     g.attempts = g_attempts.p;
     g.capacity = photon_cap;
     return s;
@@ -489,8 +494,8 @@ void size_wavefronts(pale_handle* h, uint64_t all_pix, uint32_t max_pix) {
     h->cg_paths.alloc(h->path_cap); h->cg_paths2.alloc(h->path_cap);
     h->cg_qrec.alloc(2 * (size_t)kGatherHits * h->path_cap); h->cg_res.alloc(h->path_cap);
     h->cg_info_a.alloc(h->path_cap); h->cg_info_b.alloc(h->path_cap);
-    h->cg_mhit.alloc(h->path_cap); h->cg_walk.alloc(2 * (size_t)h->path_cap);
-    h->cg_khit.alloc((size_t)kKHitWords * h->path_cap);
+    h->cg_entry.alloc(std::max<size_t>(3 + kKHitWords / 4, (3 * kGatherHits + 3) / 4) * (size_t)h->path_cap);
+    h->cg_bins.ensure(gather_bins(h->path_cap));
   }
   h->cg_fb.ensure(std::max<uint64_t>(all_pix, 1));
 }
@@ -702,6 +707,10 @@ void setup_scene(pale_handle* h, const pale_scene_desc* d) {
   h->g_scan_temp.alloc(scan_temp_words(h->cells + 1));
   h->g_stored.alloc(1);
   h->g_attempts.alloc(1);
+  const size_t lit_words = (size_t)h->res[1] * h->res[2] * (((size_t)h->res[0] + 31) / 32);
+  h->g_lit.alloc(lit_words);
+  h->g_lit_x.alloc(lit_words);
+  CK(cudaMemsetAsync(h->g_lit.p, 0, lit_words * 4, s));   // no photons yet
   h->cam_cursor.alloc(1);
   CK(cudaMemsetAsync(h->cam_cursor.p, 0, 4, s));
   CK(cudaMemsetAsync(h->g_stored.p, 0, 4, s));
@@ -935,6 +944,8 @@ void trace_photon_map(pale_handle* h) {
   G.pc = h->g_pc.p;
   G.d_stored = h->g_stored.p;
   G.d_attempts = h->g_attempts.p;
+  G.lit_x = h->g_lit_x.p;
+  G.lit = h->g_lit.p;
   grid_build(P.scene, h->run.p, P.ps, G, h->cells, h->key_bits, s);
   CK(cudaMemcpyAsync(h->cam_cursor.p, &h->run.p->seed_cursor, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   ++h->photon_gen;
@@ -998,9 +1009,13 @@ FrameArgs frame_args(const std::vector<pale_handle*>& scenes, uint32_t nsel, uin
   F.qrec = h->cg_qrec.p;
   F.info_a = h->cg_info_a.p;
   F.info_b = h->cg_info_b.p;
-  F.mhit = h->cg_mhit.p;
-  F.walk = h->cg_walk.p;
-  F.khit = h->cg_khit.p;
+  F.mhit = h->cg_entry.p;
+  F.walk = F.mhit + h->path_cap;
+  F.khit = reinterpret_cast<uint32_t*>(F.walk + 2 * (size_t)h->path_cap);
+  F.rec_bin = reinterpret_cast<uint2*>(h->cg_entry.p);
+  F.rec_order = reinterpret_cast<uint32_t*>(F.rec_bin + (size_t)kGatherHits * h->path_cap);
+  F.rec_heavy = reinterpret_cast<uint32_t*>(F.rec_bin);
+  F.bins = h->cg_bins.p;
   F.counts = h->cg_counts.p;
   F.res = h->cg_res.p;
   F.fb = h->cg_fb.p;
@@ -2302,7 +2317,7 @@ int pale_load_photons(pale_handle* h, uint32_t n, const float* pos, const float*
     G.cell_id = h->g_cell_id.p; G.sorted = h->g_sorted.p; G.keys_tmp = h->g_keys.p; G.vals_tmp = h->g_vals_tmp.p;
     G.sort_temp = h->g_sort_temp.p; G.cell_count = h->g_cell_count.p; G.cell_off = h->g_cell_off.p;
     G.scan_temp = h->g_scan_temp.p; G.pa = h->g_pa.p; G.pb = h->g_pb.p; G.pc = h->g_pc.p; G.d_stored = h->g_stored.p;
-    G.d_attempts = h->g_attempts.p;
+    G.d_attempts = h->g_attempts.p; G.lit_x = h->g_lit_x.p; G.lit = h->g_lit.p;
     grid_build(h->view(), h->run.p, ps, G, h->cells, h->key_bits, s);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));

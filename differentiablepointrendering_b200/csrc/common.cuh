@@ -188,6 +188,10 @@ struct LightView {
   const uint32_t* tri;     // per emissive triangle global triangle id
 };
 
+// A lookup's window of grid cells is at most this wide in every axis, up to
+// rounding (the radius is two cells).
+constexpr int kLitCells = 5;
+
 struct GridView {
   float radius;
   V3 origin;
@@ -198,6 +202,8 @@ struct GridView {
   const float4* pa;           // sorted: position, power.r
   const float4* pb;           // sorted: incoming direction, power.g
   const float* pc;            // sorted: power.b
+  const uint32_t* lit;        // bit per cell c: some cell of [c, c + kLitCells) holds a photon
+  uint32_t lit_row;           // words of a row of bits (fixed y, z)
   const uint32_t* attempts;   // deposits attempted (device)
   uint64_t capacity;
 };
@@ -231,6 +237,8 @@ struct RunState {
   uint32_t event_count;     // events of the current bounce
   uint32_t error;
   uint32_t walk_next;       // next ray of a persistent walk (sorted position)
+  uint32_t lookup_next;     // lookups of the current round that find photons
+  uint32_t heavy_next;      // those of them that scan many photons
   unsigned long long photon_segments;
   unsigned long long gather_segments;
   unsigned long long adjoint_segments;

@@ -138,6 +138,8 @@ struct GridBufs {
   float* pc;
   uint32_t* d_stored;     // photons stored (device)
   uint32_t* d_attempts;   // deposits attempted, read by the lookups
+  uint32_t* lit_x;        // the lit bits of GridView and their first pass
+  uint32_t* lit;
 };
 
 // Adjoint pending interaction per path (PendingAdjointState,
@@ -262,6 +264,16 @@ struct FrameArgs {
   float4* mhit;
   float4* walk;
   uint32_t* khit;
+  // the round's lookups, written once the walk's buffers above have been
+  // read, in their memory: per record its bin (a group of grid cells) and
+  // its rank in the bin, and the records to look up, in bin order; bins is
+  // a power of two of counters, then offsets.  rec_heavy, the records left
+  // to the heavy lookups, takes the place of rec_bin.
+  uint2* rec_bin;
+  uint32_t* rec_order;
+  uint32_t* rec_heavy;
+  uint32_t* bins;
+  uint32_t bin_mask;       // bins - 1 (set per round)
   KernelTimer* timer;      // host side, may be null
   // host side: a pinned word the length of the next round's queue is copied
   // to, and the event behind that copy
@@ -314,6 +326,10 @@ constexpr int kRoundMinBlocks = PALE_ROUND_MIN_BLOCKS;
 #define PALE_LOOKUP_MIN_BLOCKS 4
 #endif
 constexpr int kLookupMinBlocks = PALE_LOOKUP_MIN_BLOCKS;
+#ifndef PALE_HEAVY_MIN_BLOCKS
+#define PALE_HEAVY_MIN_BLOCKS 6
+#endif
+constexpr int kHeavyMinBlocks = PALE_HEAVY_MIN_BLOCKS;
 // The persistent walks (adjoint closest hit, camera 8 hits): lanes whose
 // walk has ended take a new ray every PALE_REFILL_STEPS node visits;
 // PALE_WALK_MIN_BLOCKS is the adjoint walk's register budget.
@@ -338,6 +354,11 @@ constexpr int kWalkMinBlocks = PALE_WALK_MIN_BLOCKS;
 #define PALE_TRANSPORT_MIN_BLOCKS 3
 #endif
 constexpr int kTransportMinBlocks = PALE_TRANSPORT_MIN_BLOCKS;
+
+// Bins a round's lookup records are grouped into: the grid cell modulo a
+// power of two, at most kMaxBins (32 MB of counters, within L2).
+constexpr uint32_t kMinBins = 1u << 11;
+constexpr uint32_t kMaxBins = 1u << 23;
 
 // Per-camera L2 loss 0.5 mean((ldr - target)^2) over the RGB values of
 // each camera of a finished frame (needs a.ldr and a.target), summed in
@@ -471,6 +492,9 @@ struct SweepArgs {
 };
 void gather_backward(const FrameArgs& a, const std::vector<CameraRec>& views, const VertexPlan& plan,
                      const SweepArgs& w, const VertexStore& scratch, cudaStream_t s);
+// Bins of a gather round of at most `entries` queue entries (two per
+// entry, a power of two).
+uint32_t gather_bins(uint32_t entries);
 void adjoint_raygen(const AdjointArgs& a, uint32_t npaths, cudaStream_t s);
 void adjoint_bounce(const AdjointArgs& a, uint32_t bounce, uint32_t npaths, cudaStream_t s);
 

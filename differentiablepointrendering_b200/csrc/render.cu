@@ -349,6 +349,40 @@ __global__ void k_gather_sorted(const uint32_t* __restrict__ sorted, const uint3
   sc[i] = c[j];
 }
 
+// The lit bits of GridView: k_lit_x a row's occupied cells, each spread over
+// the kLitCells - 1 cells before it in x (a warp per word: its 32 cells and
+// the first of the next), k_lit_yz the spread in y and z.
+__global__ void __launch_bounds__(kBlock) k_lit_x(GridView G, uint32_t* __restrict__ out) {
+  const size_t w = ((size_t)blockIdx.x * kBlock + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const size_t words = (size_t)G.res[1] * G.res[2] * G.lit_row;
+  if (w >= words) return;
+  const size_t row = w / G.lit_row;
+  const uint32_t x0 = (uint32_t)(w - row * G.lit_row) * 32u;
+  const uint32_t* off = G.cell_off + row * G.res[0];
+  auto occupied = [&](uint32_t x) { return x < (uint32_t)G.res[0] && __ldg(&off[x + 1]) > __ldg(&off[x]); };
+  const uint32_t lo = __ballot_sync(0xffffffffu, occupied(x0 + lane));
+  const uint32_t hi = __ballot_sync(0xffffffffu, lane < kLitCells - 1 && occupied(x0 + 32 + lane));
+  if (lane) return;
+  uint32_t bits = 0;
+#pragma unroll
+  for (int k = 0; k < kLitCells; ++k) bits |= __funnelshift_r(lo, hi, k);
+  out[w] = bits;
+}
+
+__global__ void __launch_bounds__(kBlock) k_lit_yz(GridView G, const uint32_t* __restrict__ in,
+                                                   uint32_t* __restrict__ out) {
+  const size_t w = (size_t)blockIdx.x * kBlock + threadIdx.x;
+  if (w >= (size_t)G.res[1] * G.res[2] * G.lit_row) return;
+  const size_t row = w / G.lit_row;
+  const int y = (int)(row % G.res[1]), z = (int)(row / G.res[1]);
+  uint32_t bits = 0;
+  for (int k = 0; k < kLitCells && z + k < G.res[2]; ++k)
+    for (int j = 0; j < kLitCells && y + j < G.res[1]; ++j)
+      bits |= in[w + ((size_t)k * G.res[1] + j) * G.lit_row];
+  out[w] = bits;
+}
+
 void grid_build(const SceneView& sv, RunState* st, const PhotonStore& ps, const GridBufs& g, uint32_t cells,
                 int key_bits, cudaStream_t s) {
   const uint32_t cap = (uint32_t)ps.capacity;
@@ -361,6 +395,9 @@ void grid_build(const SceneView& sv, RunState* st, const PhotonStore& ps, const 
   exclusive_scan(g.cell_count, g.cell_off, cells + 1, g.scan_temp, nullptr, s);
   radix_sort_pairs(sort_keys, g.sorted, sort_keys_tmp, g.vals_tmp, g.d_stored, cap, key_bits, g.sort_temp, s);
   k_gather_sorted<<<blocks_for(cap), kBlock, 0, s>>>(g.sorted, g.d_stored, ps.a, ps.b, ps.c, g.pa, g.pb, g.pc); note_launch();
+  const uint64_t words = (uint64_t)sv.grid.res[1] * sv.grid.res[2] * sv.grid.lit_row;
+  k_lit_x<<<blocks_for(words * 32), kBlock, 0, s>>>(sv.grid, g.lit_x); note_launch();
+  k_lit_yz<<<blocks_for(words), kBlock, 0, s>>>(sv.grid, g.lit_x, g.lit); note_launch();
 }
 
 // ---------------------------------------------------------- primary rays
@@ -492,7 +529,7 @@ __device__ __forceinline__ uint32_t vs_ent_slot(const FrameArgs& A, uint32_t rou
 // mesh distance plus intersect_scene's margin.
 __global__ void k_cg_mesh(FrameArgs A, uint32_t round) {
   const uint32_t n = A.counts[round];
-  if (blockIdx.x == 0 && threadIdx.x == 0) A.st->walk_next = 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) A.st->walk_next = A.st->lookup_next = A.st->heavy_next = 0u;
   const RayRec* __restrict__ in = A.paths[round & 1];
   for (uint32_t slot = blockIdx.x * kBlock + threadIdx.x; slot < n; slot += gridDim.x * kBlock) {
     const float4 ro = in[slot].o;
@@ -756,54 +793,212 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_cg_round(FrameArgs 
   warp_count(&A.st->gather_segments, segs);
 }
 
-// Round step 2: one warp per lookup record (warps stride over the records,
-// so in deep rounds every lookup has a warp of its own).  Lane 0 writes the
-// layer's contribution Lo * weight over the record's first float4.
+// Round step 2: the photon lookups of the round's records.  Most layers see
+// no photon at all (on a lit box of 200k surfels 68% of the camera lookups,
+// the cloud being dark away from the light) and most photons are scanned by
+// the few lookups near the light (95% of them by lookups of more than 256
+// photons), so the records are split three ways:
+// - k_cg_lit (a thread per record) finishes those whose window holds no
+//   photon, from one bit per grid cell, and lists the others, in the order
+//   of their grid cells when there are enough of them to share photons: a
+//   counting sort into bins (the cell modulo the number of bins; a record's
+//   rank in its bin is the counter it found), k_bin_offsets making offsets
+//   of the counts and k_cg_order placing the records;
+// - k_cg_lookup does the short ones, kLookupLanes lanes each, and lists
+//   those of more than kLookupHeavy photons;
+// - k_cg_lookup_heavy does these, a warp each.
+// The order inside a bin and between blocks of bins depends on timing, the
+// results do not: each lookup reads its own window alone.  On 200k surfels x
+// 8 views the lookups of a step took 173 ms with a warp per record, 78 ms
+// so: 37 ms the heavy ones, which wait on L1 and L2 (11 TB/s of photon
+// records read by the SMs), 36 ms the short ones (63% of the issue slots),
+// 5 ms the split.
+// Queue entries of a round from which its lookups are grouped by grid cell:
+// the grouping costs three short launches (9 us when nothing is there to
+// group) and, on 200k surfels x 8 views, 4.9 ms against the 6.7 ms that the
+// shared photons save (lookups 36.9 -> 30.2 ms, the heavy ones alike).
+constexpr uint32_t kSortEntries = 32768;
+
+// The radiance a layer adds to its path: Lo * weight.
+__device__ __forceinline__ float4 layer_radiance(const SceneView& S, uint32_t kind, uint32_t idx, V3 E, float weight) {
+  const float4 refl = kind == kRecSurfel ? __ldg(&S.sf.alb[idx]) : __ldg(&S.mesh.materials[idx]);
+  V3 Lo;
+  if (kind == kRecSurfel) {
+    Lo = mul(E, scale(scale(xyz(refl), refl.w), kInvPi));
+  } else {
+    Lo = mul(scale(xyz(refl), kInvPi), E);
+  }
+  const V3 c = scale(Lo, weight);
+  return make_float4(c.x, c.y, c.z, 0.f);
+}
+
+template <bool kMulti, bool kSort>
+__global__ void __launch_bounds__(kBlock) k_cg_lit(FrameArgs A, uint32_t round) {
+  const uint32_t n = A.counts[kMaxLayers + 2 + round];
+  const int lane = threadIdx.x & 31;
+  uint32_t queries = 0;
+  for (uint32_t b = blockIdx.x * kBlock; b < n; b += gridDim.x * kBlock) {
+    const uint32_t i = b + threadIdx.x;
+    uint32_t bin = kInvalid;
+    if (i < n) {
+      const float4 rb = A.qrec[2 * (size_t)i + 1];
+      const uint32_t word = __float_as_uint(rb.w), kind = word >> 30;
+      if (kind != kRecNone) {
+        const float4 ra = A.qrec[2 * (size_t)i];
+        const uint32_t sid = kMulti ? (word >> 27) & 7u : 0u;
+        const SceneView& S = A.scenes.s[sid];
+        ++queries;
+        if (window_lit(S.grid, xyz(ra))) {
+          bin = 0;
+          if (kSort) {
+            int c[3];
+            world_to_cell(S.grid, xyz(ra), c);
+            bin = ((uint32_t)((c[2] * S.grid.res[1] + c[1]) * S.grid.res[0] + c[0]) + sid * 0x9E3779B1u) & A.bin_mask;
+          }
+        } else {
+          const V3 E = v3(0.f, 0.f, 0.f);
+          A.qrec[2 * (size_t)i] = layer_radiance(S, kind, word & kRecIndexMask, E, ra.w);
+          const uint32_t vr = vs_rec_slot(A, round, i);
+          if (vr != kInvalid) A.vs.rec_ew[vr] = make_float4(0.f, 0.f, 0.f, rb.w);
+        }
+      }
+    }
+    if (kSort) {
+      // one atomic per bin present in the warp: a view that looks at one
+      // spot puts most of its records into few bins
+      const unsigned peers = __match_any_sync(0xffffffffu, bin);
+      const int leader = __ffs(peers) - 1;
+      uint32_t base = 0;
+      if (lane == leader && bin != kInvalid) base = atomicAdd(&A.bins[bin], (uint32_t)__popc(peers));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (i < n) A.rec_bin[i] = make_uint2(bin, base + __popc(peers & ((1u << lane) - 1u)));
+    } else {
+      const unsigned lit = __ballot_sync(0xffffffffu, bin != kInvalid);
+      uint32_t base = 0;
+      if (lit && lane == 0) base = atomicAdd(&A.st->lookup_next, (uint32_t)__popc(lit));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (bin != kInvalid) A.rec_order[base + __popc(lit & ((1u << lane) - 1u))] = i;
+    }
+  }
+  warp_count(&A.st->gather_queries, queries);
+}
+
+// Counts -> offsets: every block scans its kBlock * kBinItems bins and takes
+// its range of the order with one atomic.
+constexpr int kBinItems = 8;
+__global__ void __launch_bounds__(kBlock) k_bin_offsets(uint32_t* __restrict__ bins, uint32_t* __restrict__ next) {
+  __shared__ uint32_t s_warp[kBlock / 32];
+  __shared__ uint32_t s_base;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint4* p = reinterpret_cast<uint4*>(bins) + ((size_t)blockIdx.x * kBlock + threadIdx.x) * (kBinItems / 4);
+  uint4 v[kBinItems / 4];
+  uint32_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < kBinItems / 4; ++k) {
+    v[k] = p[k];
+    sum += v[k].x + v[k].y + v[k].z + v[k].w;
+  }
+  uint32_t x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s_warp[wid] = x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t t = 0;
+    for (int w = 0; w < kBlock / 32; ++w) {
+      const uint32_t c = s_warp[w];
+      s_warp[w] = t;
+      t += c;
+    }
+    s_base = t ? atomicAdd(next, t) : 0u;
+  }
+  __syncthreads();
+  uint32_t run = s_base + s_warp[wid] + x - sum;
+#pragma unroll
+  for (int k = 0; k < kBinItems / 4; ++k) {
+    const uint4 c = v[k];
+    p[k] = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
+    run += c.x + c.y + c.z + c.w;
+  }
+}
+
+__global__ void __launch_bounds__(kBlock) k_cg_order(FrameArgs A, uint32_t round) {
+  const uint32_t n = A.counts[kMaxLayers + 2 + round];
+  for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
+    const uint2 b = A.rec_bin[i];
+    if (b.x != kInvalid) A.rec_order[A.bins[b.x] + b.y] = i;
+  }
+}
+
+// A group's first lane writes the layer's contribution over the record's
+// first float4.
 template <bool kMulti>
 __global__ void __launch_bounds__(kBlock, kLookupMinBlocks) k_cg_lookup(FrameArgs A, uint32_t round) {
-  __shared__ float4 s_terms[kBlock];
+  __shared__ uint32_t s_list[kBlock / kLookupLanes][kLookupList];
+  __shared__ float s_sq[kBlock / kLookupLanes][16];
   __shared__ GatherConst s_gc[kMaxScenes];
   if (threadIdx.x < A.scenes.n) s_gc[threadIdx.x] = gather_const(A.scenes.s[threadIdx.x].grid);
   __syncthreads();
-  const uint32_t n = A.counts[kMaxLayers + 2 + round];
-  const int lane = threadIdx.x & 31;
-  float4* terms = s_terms + (threadIdx.x & ~31u);
-  const uint32_t warps = gridDim.x * (kBlock / 32);
-  uint32_t queries = 0, scanned = 0;
-  // lanes 0-7 hold the 8 floats of the next record, loaded one record ahead
-  uint32_t i = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
-  float pre = (i < n && lane < 8) ? reinterpret_cast<const float*>(A.qrec + 2 * (size_t)i)[lane] : 0.f;
-  for (; i < n; i += warps) {
-    const float cur = pre;
-    if (i + warps < n && lane < 8) pre = reinterpret_cast<const float*>(A.qrec + 2 * (size_t)(i + warps))[lane];
-    auto field = [&](int f) { return __shfl_sync(0xffffffffu, cur, f); };
-    const float4 ra = make_float4(field(0), field(1), field(2), field(3));
-    const float4 rb = make_float4(field(4), field(5), field(6), field(7));
+  const uint32_t n = A.st->lookup_next;
+  const uint32_t g = threadIdx.x / kLookupLanes, groups = gridDim.x * (kBlock / kLookupLanes);
+  uint32_t scanned = 0;
+  for (uint32_t b = blockIdx.x * (kBlock / kLookupLanes) + g; __any_sync(0xffffffffu, b < n); b += groups) {
+    const bool valid = b < n;
+    uint32_t i = 0;
+    float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rb = ra;
+    if (valid) {
+      i = A.rec_order[b];
+      ra = A.qrec[2 * (size_t)i];
+      rb = A.qrec[2 * (size_t)i + 1];
+    }
     const uint32_t word = __float_as_uint(rb.w);
-    const uint32_t kind = word >> 30, idx = word & kRecIndexMask, sid = kMulti ? (word >> 27) & 7u : 0u;
-    if (kind == kRecNone) continue;
+    const uint32_t sid = kMulti ? (word >> 27) & 7u : 0u;
     const SceneView& S = A.scenes.s[sid];
-    // the reflectance, loaded before the gather so that its latency overlaps it
-    float4 refl = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (lane == 0) refl = kind == kRecSurfel ? __ldg(&S.sf.alb[idx]) : __ldg(&S.mesh.materials[idx]);
     uint32_t cnt = 0;
-    const V3 E = gather_irradiance_warp<false>(S.grid, s_gc[sid], xyz(ra), xyz(rb), terms, cnt);
-    if (lane == 0) {
-      ++queries;
-      scanned += cnt;
-      V3 Lo;
-      if (kind == kRecSurfel) {
-        Lo = mul(E, scale(scale(xyz(refl), refl.w), kInvPi));
+    bool heavy;
+    const V3 E = gather_irradiance_lanes<kLookupLanes>(S.grid, s_gc[sid], xyz(ra), xyz(rb), valid, s_list[g],
+                                                       s_sq[g], cnt, heavy);
+    if (valid && threadIdx.x % kLookupLanes == 0) {
+      if (heavy) {
+        A.rec_heavy[atomicAdd(&A.st->heavy_next, 1u)] = i;
       } else {
-        Lo = mul(scale(xyz(refl), kInvPi), E);
+        scanned += cnt;
+        A.qrec[2 * (size_t)i] = layer_radiance(S, word >> 30, word & kRecIndexMask, E, ra.w);
+        const uint32_t vr = vs_rec_slot(A, round, i);
+        if (vr != kInvalid) A.vs.rec_ew[vr] = make_float4(E.x, E.y, E.z, rb.w);
       }
-      const V3 c = scale(Lo, ra.w);
-      A.qrec[2 * (size_t)i] = make_float4(c.x, c.y, c.z, 0.f);
+    }
+  }
+  warp_count(&A.st->photons_scanned, scanned);
+  warp_count(&A.st->gather_photons_scanned, scanned);
+}
+
+template <bool kMulti>
+__global__ void __launch_bounds__(kBlock, kHeavyMinBlocks) k_cg_lookup_heavy(FrameArgs A, uint32_t round) {
+  __shared__ GatherConst s_gc[kMaxScenes];
+  if (threadIdx.x < A.scenes.n) s_gc[threadIdx.x] = gather_const(A.scenes.s[threadIdx.x].grid);
+  __syncthreads();
+  const uint32_t n = A.st->heavy_next;
+  const int lane = threadIdx.x & 31;
+  uint32_t scanned = 0;
+  for (uint32_t b = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); b < n; b += gridDim.x * (kBlock / 32)) {
+    const uint32_t i = A.rec_heavy[b];
+    const float4 ra = A.qrec[2 * (size_t)i], rb = A.qrec[2 * (size_t)i + 1];
+    const uint32_t word = __float_as_uint(rb.w);
+    const uint32_t sid = kMulti ? (word >> 27) & 7u : 0u;
+    const SceneView& S = A.scenes.s[sid];
+    uint32_t cnt = 0;
+    const V3 E = gather_irradiance_rows(S.grid, s_gc[sid], xyz(ra), xyz(rb), cnt);
+    if (lane == 0) {
+      scanned += cnt;
+      A.qrec[2 * (size_t)i] = layer_radiance(S, word >> 30, word & kRecIndexMask, E, ra.w);
       const uint32_t vr = vs_rec_slot(A, round, i);
       if (vr != kInvalid) A.vs.rec_ew[vr] = make_float4(E.x, E.y, E.z, rb.w);
     }
   }
-  warp_count(&A.st->gather_queries, queries);
   warp_count(&A.st->photons_scanned, scanned);
   warp_count(&A.st->gather_photons_scanned, scanned);
 }
@@ -925,6 +1120,12 @@ void image_loss(const FrameArgs& a, double* partials, double* loss, cudaStream_t
   k_loss_final<<<(a.ncams + 63) / 64, 64, 0, s>>>(a, partials, kLossChunks, loss); note_launch();
 }
 
+uint32_t gather_bins(uint32_t entries) {
+  uint32_t b = kMinBins;
+  while (b < kMaxBins && b < 2ull * entries) b <<= 1;
+  return b;
+}
+
 std::vector<GatherChunk> gather_chunks(const std::vector<CameraRec>& views, uint32_t path_capacity) {
   const size_t nv = views.size();
   std::vector<GatherChunk> out;
@@ -981,7 +1182,7 @@ namespace {
 
 // The launch shapes of the camera gather's kernels.
 struct GatherShape {
-  uint32_t grid_r = 1, grid_l = 1;
+  uint32_t grid_r = 1, grid_l = 1, grid_h = 1, grid_b = 1;
   int wt = kBlock;
   size_t smem = 0;
 };
@@ -990,7 +1191,7 @@ template <bool kMulti>
 GatherShape gather_shape(const FrameArgs& a) {
   GatherShape g;
   // persistent grids: every SM filled once
-  int dev = 0, sms = 148, per_sm_l = 1, per_sm_r = 1;
+  int dev = 0, sms = 148, per_sm_l = 1, per_sm_h = 1, per_sm_r = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   g.wt = a.walk_block == 64 || a.walk_block == 128 ? (int)a.walk_block : kBlock;
@@ -999,13 +1200,16 @@ GatherShape gather_shape(const FrameArgs& a) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_l, k_cg_lookup<kMulti>, kBlock, 0);
   g.grid_r = (uint32_t)std::max(1, sms * std::max(1, per_sm_r));
   g.grid_l = (uint32_t)std::max(1, sms * std::max(1, per_sm_l));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_h, k_cg_lookup_heavy<kMulti>, kBlock, 0);
+  g.grid_h = (uint32_t)std::max(1, sms * std::max(1, per_sm_h));
+  g.grid_b = (uint32_t)std::max(1, sms * 8);
   return g;
 }
 
 // The rounds of one chunk of n paths (its view_start already on the
 // device); returns the rounds run.
 template <bool kMulti>
-uint32_t gather_rounds(const FrameArgs& a, const GatherShape& g, uint32_t n, cudaStream_t s) {
+uint32_t gather_rounds(FrameArgs a, const GatherShape& g, uint32_t n, cudaStream_t s) {
   cudaMemsetAsync(a.counts, 0, 2 * (kMaxLayers + 2) * sizeof(uint32_t), s);
   k_cg_init<<<blocks_for(n), kBlock, 0, s>>>(a, n); note_launch();
   // every round consumes at least one layer of each live path, so
@@ -1026,7 +1230,17 @@ uint32_t gather_rounds(const FrameArgs& a, const GatherShape& g, uint32_t n, cud
     cudaMemcpyAsync(const_cast<uint32_t*>(a.h_live), a.counts + round + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     cudaEventRecord(a.round_ev, s);
     if (a.timer) a.timer->begin(kTimeLookup, s);
+    if (live >= kSortEntries) {
+      a.bin_mask = gather_bins(live) - 1u;
+      cudaMemsetAsync(a.bins, 0, ((size_t)a.bin_mask + 1) * sizeof(uint32_t), s);
+      k_cg_lit<kMulti, true><<<g.grid_b, kBlock, 0, s>>>(a, round); note_launch();
+      k_bin_offsets<<<(a.bin_mask + 1u) / (kBlock * kBinItems), kBlock, 0, s>>>(a.bins, &a.st->lookup_next); note_launch();
+      k_cg_order<<<g.grid_b, kBlock, 0, s>>>(a, round); note_launch();
+    } else {
+      k_cg_lit<kMulti, false><<<std::min(g.grid_b, blocks_for((uint64_t)live * kGatherHits)), kBlock, 0, s>>>(a, round); note_launch();
+    }
     k_cg_lookup<kMulti><<<g.grid_l, kBlock, 0, s>>>(a, round); note_launch();
+    k_cg_lookup_heavy<kMulti><<<g.grid_h, kBlock, 0, s>>>(a, round); note_launch();
     if (a.timer) a.timer->end(s);
     k_cg_compose<<<blocks_for(live), kBlock, 0, s>>>(a, round); note_launch();
     ++round;
@@ -1715,9 +1929,9 @@ void gather_backward(const FrameArgs& a0, const std::vector<CameraRec>& views, c
 // launchAdjointTransportKernel (AdjointKernels.cpp:389-509).  A warp takes
 // the events of a tile of 32 (warps stride over the tiles), lane i the
 // i-th: every lane loads its own event record (one coalesced load), the
-// warp does the photon lookups of the tile's events one after another
-// (gather_irradiance_warp, each lookup's 32 photon rounds spread over the
-// lanes) and the lane of each event keeps its irradiance; then every lane
+// warp does the photon lookups of the tile's events that have a photon in
+// reach one after another (gather_irradiance_warp, each lookup's 32 photon
+// rounds spread over the lanes) and the lane of each event keeps its irradiance; then every lane
 // evaluates its own event's terms (the opacity term as the reference
 // computes it; with gradients = "all" also the other six groups) at the
 // same time.  Events with the same target surfel are added up inside the
@@ -1737,12 +1951,16 @@ __global__ void __launch_bounds__(kBlock, kTransportMinBlocks) k_transport(Adjoi
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float4* terms = s_terms + (threadIdx.x & ~31u);
   const uint32_t warps = gridDim.x * (kBlock / 32);
-  const uint32_t tiles = (count + 31u) / 32u;
+  // a tile is 32 events, or fewer while that leaves warps without one (a
+  // tile's lookups run after one another)
+  uint32_t per = 32u;
+  while (per > 2u && count < per * warps) per >>= 1;
+  const uint32_t tiles = (count + per - 1u) / per;
   const int nterms = A.all_grads ? kTransportTerms + 1 : 1;
   uint32_t events = 0, queries = 0, scanned = 0;
   for (uint32_t tile = blockIdx.x * (kBlock / 32) + wid; tile < tiles; tile += warps) {
-    const uint32_t e = tile * 32u + lane;
-    const bool valid = e < count;
+    const uint32_t e = tile * per + lane;
+    const bool valid = lane < per && e < count;
     // the lookup's point and normal and the event's kind and indices now;
     // the throughput (and the alpha-gradient point) after the lookups
     const EventRec* src = A.ev.list + (valid ? e : 0u);
@@ -1764,8 +1982,10 @@ __global__ void __launch_bounds__(kBlock, kTransportMinBlocks) k_transport(Adjoi
     // materials[0xFFFFFFFF], AdjointKernels.cpp:446-447): no contribution
     const bool need =
         valid && (kind == kKindProjection || kind == kKindReflect || (kind == kKindNull && ev.d.z != kInvalid));
+    if (need) ++queries;
     V3 E = v3(0.f, 0.f, 0.f);
-    for (unsigned m = __ballot_sync(0xffffffffu, need); m; m &= m - 1u) {
+    const bool lit = need && window_lit(A.scenes.s[sid].grid, xyz(ev.a));
+    for (unsigned m = __ballot_sync(0xffffffffu, lit); m; m &= m - 1u) {
       const int j = __ffs(m) - 1;
       const V3 xj = v3(__shfl_sync(0xffffffffu, ev.a.x, j), __shfl_sync(0xffffffffu, ev.a.y, j),
                        __shfl_sync(0xffffffffu, ev.a.z, j));
@@ -1773,11 +1993,10 @@ __global__ void __launch_bounds__(kBlock, kTransportMinBlocks) k_transport(Adjoi
                        __shfl_sync(0xffffffffu, ev.b.z, j));
       const uint32_t sj = __shfl_sync(0xffffffffu, sid, j);
       uint32_t cnt = 0;
-      const V3 Ej = gather_irradiance_warp<true>(A.scenes.s[sj].grid, s_gc[sj], xj, nj, terms, cnt);
+      const V3 Ej = gather_irradiance_warp(A.scenes.s[sj].grid, s_gc[sj], xj, nj, terms, cnt);
       if (lane == j) {
         E = Ej;
         scanned += cnt;
-        ++queries;
       }
     }
     // this lane's event
@@ -2008,8 +2227,8 @@ void trace_transmittance(const SceneView& sv, RunState* st, uint32_t n, const fl
   note_launch();
 }
 
-__global__ void k_gather_points(SceneView S, uint32_t n, const float* __restrict__ p, const float* __restrict__ nrm,
-                                float* E) {
+__global__ void __launch_bounds__(kBlock) k_gather_points(SceneView S, uint32_t n, const float* __restrict__ p,
+                                                          const float* __restrict__ nrm, float* E) {
   __shared__ float4 s_terms[kBlock];
   const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -2020,7 +2239,7 @@ __global__ void k_gather_points(SceneView S, uint32_t n, const float* __restrict
     x = v3(p[3 * i], p[3 * i + 1], p[3 * i + 2]);
     nv = v3(nrm[3 * i], nrm[3 * i + 1], nrm[3 * i + 2]);
   }
-  unsigned qm = __ballot_sync(0xffffffffu, in);
+  unsigned qm = __ballot_sync(0xffffffffu, in && window_lit(S.grid, x));
   while (qm) {
     const int src = __ffs(qm) - 1;
     qm &= qm - 1u;
@@ -2029,7 +2248,7 @@ __global__ void k_gather_points(SceneView S, uint32_t n, const float* __restrict
     const V3 qv = v3(__shfl_sync(0xffffffffu, nv.x, src), __shfl_sync(0xffffffffu, nv.y, src),
                      __shfl_sync(0xffffffffu, nv.z, src));
     uint32_t cnt = 0;
-    const V3 r = gather_irradiance_warp<false>(S.grid, GC, qx, qv, s_terms + (threadIdx.x & ~31u), cnt);
+    const V3 r = gather_irradiance_warp(S.grid, GC, qx, qv, s_terms + (threadIdx.x & ~31u), cnt);
     if (lane == src) e = r;
   }
   if (!in) return;
