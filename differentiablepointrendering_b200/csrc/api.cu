@@ -226,7 +226,8 @@ struct pale_handle {
   DBuf<float4> adj_walkq;  // walk record per sorted position (2 float4)
   // adjoint batches
   uint32_t adj_cap = 0;
-  DBuf<uint32_t> adj_keys, adj_perm, adj_keys_tmp, adj_perm_tmp, adj_sort_temp;   // ray order of a bounce
+  DBuf<uint2> ray_at;        // the walk's order of a bounce's rays: bin and rank per queue slot
+  DBuf<uint32_t> ray_bins;
   DBuf<AdjJob> d_jobs;
   DBuf<CameraRec> d_adj_cams;
   DBuf<uint32_t> job_count, job_start;
@@ -476,9 +477,8 @@ void size_wavefronts(pale_handle* h, uint64_t all_pix, uint32_t max_pix) {
   if (adj_cap > h->adj_cap) {
     h->adj_cap = adj_cap;
     const size_t qa = std::max<size_t>(qc, h->adj_cap);
-    h->adj_keys.alloc(h->adj_cap); h->adj_perm.alloc(h->adj_cap);
-    h->adj_keys_tmp.alloc(h->adj_cap); h->adj_perm_tmp.alloc(h->adj_cap);
-    h->adj_sort_temp.alloc(radix_temp_words(h->adj_cap));
+    h->ray_at.alloc(h->adj_cap);
+    h->ray_bins.ensure((size_t)1 << ray_bins_log2(h->adj_cap));
     size_queues(h, qa);
     h->pend_a.alloc(qa); h->pend_b.alloc(qa); h->pend_c.alloc(qa);
     h->ev_stage.alloc(qa); h->ev_list.alloc(qa);
@@ -1343,12 +1343,6 @@ void adjoint_views(const std::vector<pale_handle*>& scenes, const std::vector<Vi
   A.light0_valid = h->n_lights > 0;
   A.light0_area = h->light0_area;
   A.timer = &h->timer;
-  A.sort_keys = h->adj_keys.p;
-  A.perm = h->adj_perm.p;
-  A.sort_keys_tmp = h->adj_keys_tmp.p;
-  A.perm_tmp = h->adj_perm_tmp.p;
-  A.sort_temp = h->adj_sort_temp.p;
-  A.sort_capacity = h->adj_cap;
   A.hits = h->adj_hits.p;
   A.walkq = h->adj_walkq.p;
   A.walk_block = st.walk_block;
@@ -1392,7 +1386,9 @@ void adjoint_views(const std::vector<pale_handle*>& scenes, const std::vector<Vi
     A.njobs = j1 - j0;
     const uint32_t npaths = batches[bi].second;
     adjoint_raygen(A, npaths, s);
-    for (uint32_t b = 0; b < max_depth; ++b) adjoint_bounce(A, b, npaths, s);
+    const int bins = ray_bins_log2(npaths);
+    A.rb = RayBins{bins ? h->ray_bins.p : nullptr, h->ray_at.p, bins};
+    for (uint32_t b = 0; b < max_depth; ++b) adjoint_bounce(A, b, b + 1 == max_depth, npaths, s);
   }
   CK(cudaEventRecord(h->ev1, s));
   CK(cudaGetLastError());

@@ -118,6 +118,17 @@ struct QueueBufs {
   uint32_t capacity;
 };
 
+// The rays of a bounce grouped for the walk: the compaction that writes a
+// queue counts its rays per bin (direction octant, then Morton code of the
+// origin) and keeps each ray's bin and its rank there; the counts become
+// offsets (k_bin_offsets), and a ray's place in the walk's order is its
+// bin's offset plus its rank.  bins null: the walk takes the queue's order.
+struct RayBins {
+  uint32_t* bins;         // 1 << log2 counters, then offsets
+  uint2* at;              // per queue slot: bin, rank
+  int log2;
+};
+
 struct PhotonStore {
   float4* a;              // deposit order: position, power.r
   float4* b;              // incoming direction, power.g
@@ -371,6 +382,7 @@ struct PhotonArgs {
   RunState* st;
   const uint32_t* seeds;
   QueueBufs qb;
+  RayBins rb;
   PhotonStore ps;
   uint32_t photons_per_launch;
   float inv_emitted;
@@ -397,6 +409,7 @@ struct AdjointArgs {
   RunState* st;
   const uint32_t* seeds;
   QueueBufs qb;
+  RayBins rb;
   PendingBufs pend;
   EventBufs ev;
   const float* dldi;       // packed H*W*4 per camera
@@ -415,21 +428,11 @@ struct AdjointArgs {
   uint32_t light0_valid;
   float light0_area;
   KernelTimer* timer;      // host side, may be null
-  // Bounces after the first trace their rays in the order of a sort by
-  // (direction octant, origin Morton code): thread t takes queue slot
-  // perm[t].  Each ray keeps its slot for its random stream and its
-  // outputs, so the results do not depend on the order.  Null: slot order.
-  uint32_t* sort_keys;     // 4 arrays of the queue capacity: keys, perm,
-  uint32_t* perm;          //   and the sort's ping-pong copies
-  uint32_t* sort_keys_tmp;
-  uint32_t* perm_tmp;
-  uint32_t* sort_temp;     // radix_temp_words(queue capacity)
-  uint32_t sort_capacity;
   // Per queue slot, 3 float4: the closest mesh hit (position and distance,
   // +inf on a miss; alpha, instance bits, primitive bits) and the surfel
   // walk's result (surfel bits, distance, 1 on a hit), which the mesh pass
-  // sets to no hit.  Per sorted position t (the order the walk takes the
-  // rays in), the walk's record, 2 float4: (origin, walk limit or -1 when
+  // sets to no hit.  Per position t of the walk's order (slot order, or for
+  // the bounces after the first the order of RayBins), the walk's record, 2 float4: (origin, walk limit or -1 when
   // the ray does not enter the surfel cloud's box) (unit direction, slot
   // bits).
   float4* hits;
@@ -496,7 +499,11 @@ void gather_backward(const FrameArgs& a, const std::vector<CameraRec>& views, co
 // entry, a power of two).
 uint32_t gather_bins(uint32_t entries);
 void adjoint_raygen(const AdjointArgs& a, uint32_t npaths, cudaStream_t s);
-void adjoint_bounce(const AdjointArgs& a, uint32_t bounce, uint32_t npaths, cudaStream_t s);
+// One bounce of every job of a batch; last: no bounce follows.
+void adjoint_bounce(AdjointArgs a, uint32_t bounce, bool last, uint32_t npaths, cudaStream_t s);
+// log2 of the number of ray bins of a queue of at most `rays` rays (0: too
+// few to group).
+int ray_bins_log2(uint32_t rays);
 
 // Component queries.
 void trace_rays(const SceneView& sv, RunState* st, uint32_t n, const float* o, const float* d, int32_t* inst,

@@ -16,6 +16,9 @@
 // the host loop `for (bounce...; activeCount > 0; ...)` does.
 #include "kernels.h"
 #include "trace.cuh"
+#ifndef PALE_RAY_BIN_MIN
+#define PALE_RAY_BIN_MIN 16384u
+#endif
 
 namespace pale {
 
@@ -57,13 +60,156 @@ __device__ __forceinline__ RayRec make_ray(V3 o, V3 d, V3 thr, uint32_t path, ui
   return r;
 }
 
+// --------------------------------------------------------------- binning
+// Counts -> offsets: every block scans its kBlock * kBinItems bins and takes
+// its range of the order with one atomic.
+constexpr int kBinItems = 8;
+__global__ void __launch_bounds__(kBlock) k_bin_offsets(uint32_t* __restrict__ bins, uint32_t* __restrict__ next) {
+  __shared__ uint32_t s_warp[kBlock / 32];
+  __shared__ uint32_t s_base;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint4* p = reinterpret_cast<uint4*>(bins) + ((size_t)blockIdx.x * kBlock + threadIdx.x) * (kBinItems / 4);
+  uint4 v[kBinItems / 4];
+  uint32_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < kBinItems / 4; ++k) {
+    v[k] = p[k];
+    sum += v[k].x + v[k].y + v[k].z + v[k].w;
+  }
+  uint32_t x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s_warp[wid] = x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t t = 0;
+    for (int w = 0; w < kBlock / 32; ++w) {
+      const uint32_t c = s_warp[w];
+      s_warp[w] = t;
+      t += c;
+    }
+    s_base = t ? atomicAdd(next, t) : 0u;
+  }
+  __syncthreads();
+  uint32_t run = s_base + s_warp[wid] + x - sum;
+#pragma unroll
+  for (int k = 0; k < kBinItems / 4; ++k) {
+    const uint4 c = v[k];
+    p[k] = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
+    run += c.x + c.y + c.z + c.w;
+  }
+}
+
+// The bin of this lane's item (kInvalid: none) takes it in: returns the
+// item's rank there.  Every lane of the warp calls it; one atomic per bin
+// present in the warp, since items that fall into one bin come together (a
+// view that looks at one spot, a beam of rays).
+__device__ __forceinline__ uint32_t bin_rank(uint32_t* __restrict__ bins, uint32_t bin) {
+  const int lane = threadIdx.x & 31;
+  const unsigned peers = __match_any_sync(0xffffffffu, bin);
+  const int leader = __ffs(peers) - 1;
+  uint32_t base = 0;
+  if (lane == leader && bin != kInvalid) base = atomicAdd(&bins[bin], (uint32_t)__popc(peers));
+  return __shfl_sync(0xffffffffu, base, leader) + __popc(peers & ((1u << lane) - 1u));
+}
+
+__device__ __forceinline__ uint32_t spread9(uint32_t v) {
+  v &= 0x1FFu;
+  v = (v | (v << 16)) & 0x030000FFu;
+  v = (v | (v << 8)) & 0x0300F00Fu;
+  v = (v | (v << 4)) & 0x030C30C3u;
+  v = (v | (v << 2)) & 0x09249249u;
+  return v;
+}
+
+// The bin of a ray: the leading bits of (direction octant, 27-bit Morton
+// code of the origin on a 512^3 lattice over its scene's grid box); in a
+// call of several scenes of (scene, octant, 24-bit Morton code), so that the
+// rays of one scene stay together.
+__device__ __forceinline__ uint32_t ray_bin(const GridView& G, const RayRec& ry, uint32_t sid, bool multi, int log2) {
+  uint32_t q[3];
+  const float o[3] = {ry.o.x, ry.o.y, ry.o.z}, lo[3] = {G.origin.x, G.origin.y, G.origin.z},
+              ext[3] = {G.cell.x * G.res[0], G.cell.y * G.res[1], G.cell.z * G.res[2]};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float f = (o[k] - lo[k]) / fmaxf(ext[k], 1e-30f) * 512.0f;
+    q[k] = (uint32_t)fminf(fmaxf(f, 0.0f), 511.0f);
+  }
+  const uint32_t oct = (ry.d.x < 0.f ? 1u : 0u) | (ry.d.y < 0.f ? 2u : 0u) | (ry.d.z < 0.f ? 4u : 0u);
+  const uint32_t morton = (spread9(q[0]) << 2) | (spread9(q[1]) << 1) | spread9(q[2]);
+  const uint32_t key = multi ? (sid << 27) | (oct << 24) | (morton >> 3) : (oct << 27) | morton;
+  return key >> (30 - log2);
+}
+
+__device__ __forceinline__ uint32_t ray_bin(const PhotonArgs& A, const RayRec& ry) {
+  return ray_bin(A.scene.grid, ry, 0u, false, A.rb.log2);
+}
+__device__ __forceinline__ uint32_t ray_bin(const AdjointArgs& A, const RayRec& ry) {
+  const bool multi = A.scenes.n > 1;
+  const uint32_t sid = multi ? A.cams[A.jobs[__float_as_uint(ry.d.w) >> 8].cam].scene : 0u;
+  return ray_bin(A.scenes.s[sid].grid, ry, sid, multi, A.rb.log2);
+}
+
+// Enough bins that a bin holds a few rays, at most 4 MB of counters; below
+// 16k rays the walk is shorter than the grouping.
+int ray_bins_log2(uint32_t rays) {
+  if (rays < PALE_RAY_BIN_MIN) return 0;
+  int b = 11;
+  while (b < 20 && (4u << b) < rays) ++b;
+  return b;
+}
+
 // ---------------------------------------------------------- compaction
 // One block: exclusive scan of the per-tile (alive, deposit/event) counts
-// of `n_in` slots; updates queue length, deposit/event bases and seeds.
+// of `n_in` slots; updates queue length, deposit/event bases and seeds.  The
+// adjoint launches a second block for its jobs: the queue start of every job
+// after the compaction is the exclusive scan of the survivor counts, which
+// are cleared for the bounce after next.
+struct JobScan {
+  uint32_t* count;
+  uint32_t* start;
+  uint32_t n;
+};
+
+__device__ __forceinline__ void scan_jobs(const JobScan& js, uint32_t* s_w) {
+  const uint32_t j = threadIdx.x;
+  const int lane = j & 31, wid = j >> 5;
+  const uint32_t c = j < js.n ? js.count[j] : 0u;
+  uint32_t x = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s_w[wid] = x;
+  __syncthreads();
+  if (wid == 0) {
+    uint32_t w = s_w[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    s_w[lane] = w;
+  }
+  __syncthreads();
+  js.start[j] = (wid > 0 ? s_w[wid - 1] : 0u) + x - c;
+  js.count[j] = 0u;
+}
+
+static_assert(kMaxJobsPerBatch == 1024, "scan_jobs: a thread per job");
 __global__ void __launch_bounds__(1024) k_queue_scan(RunState* st, const uint2* __restrict__ counts, uint2* __restrict__ offsets,
-                             uint32_t parity, int emission, uint32_t emission_n, int events, uint64_t photon_cap) {
+                             uint32_t parity, int emission, uint32_t emission_n, int events, uint64_t photon_cap,
+                             JobScan jobs) {
   __shared__ uint32_t s_wx[32], s_wy[32];
   __shared__ uint32_t s_carry[2];
+  if (blockIdx.x == 1) {
+    scan_jobs(jobs, s_wx);
+    return;
+  }
   const uint32_t n_in = emission ? emission_n : st->active[parity];
   const uint32_t tiles = (n_in + kBlock - 1) / kBlock;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -111,13 +257,28 @@ __global__ void __launch_bounds__(1024) k_queue_scan(RunState* st, const uint2* 
       if ((uint64_t)st->photon_base + s_carry[1] > photon_cap) atomicOr(&st->error, kErrPhotonCapacity);
     }
     st->seed_cursor += (emission || n_in > 0) ? 1u : 0u;
+    st->ray_next = 0u;
   }
 }
 
-// Compacts staged rays (and deposits or events) of the `n_in` input slots.
-template <int kMode>  // 0 photons, 1 adjoint events
-__global__ void k_queue_scatter(RunState* st, QueueBufs qb, uint32_t parity, int emission, uint32_t emission_n,
-                                PhotonStore ps, EventBufs ev) {
+// Compacts staged rays (and deposits or events) of the `n_in` input slots,
+// and takes the rays into their bins for the next bounce's walk.
+__device__ __forceinline__ void place_side(const PhotonArgs& A, uint32_t slot, uint32_t rank) {
+  const uint64_t dst = (uint64_t)A.st->photon_base + rank;
+  if (dst < A.ps.capacity) {
+    A.ps.a[dst] = A.ps.sa[slot];
+    A.ps.b[dst] = A.ps.sb[slot];
+    A.ps.c[dst] = A.ps.sc[slot];
+  }
+}
+__device__ __forceinline__ void place_side(const AdjointArgs& A, uint32_t slot, uint32_t rank) {
+  A.ev.list[rank] = A.ev.stage[slot];
+}
+
+template <class Args>   // PhotonArgs (deposits), AdjointArgs (events)
+__global__ void k_queue_scatter(Args A, uint32_t parity, int emission, uint32_t emission_n) {
+  RunState* st = A.st;
+  const QueueBufs& qb = A.qb;
   __shared__ uint32_t s_wx[kBlock / 32], s_wy[kBlock / 32];
   const uint32_t n_in = emission ? emission_n : st->active[parity];
   const uint32_t tile = blockIdx.x;
@@ -135,23 +296,22 @@ __global__ void k_queue_scatter(RunState* st, QueueBufs qb, uint32_t parity, int
   for (int w = 0; w < wid; ++w) { ra += s_wx[w]; rs += s_wy[w]; }
   const uint2 off = qb.tile_offsets[tile];
   RayRec* out = qb.q[emission ? 0u : (parity ^ 1u)];
+  uint32_t bin = kInvalid, dst = 0;
   if (alive) {
-    uint32_t dst = off.x + ra;
-    if (dst < qb.capacity) out[dst] = qb.stage[slot];
-    else flag_error(st, kErrQueueCapacity);
-  }
-  if (side) {
-    if (kMode == 0) {
-      uint64_t dst = (uint64_t)st->photon_base + off.y + rs;
-      if (dst < ps.capacity) {
-        ps.a[dst] = ps.sa[slot];
-        ps.b[dst] = ps.sb[slot];
-        ps.c[dst] = ps.sc[slot];
-      }
+    dst = off.x + ra;
+    if (dst < qb.capacity) {
+      const RayRec ry = qb.stage[slot];
+      out[dst] = ry;
+      if (A.rb.bins) bin = ray_bin(A, ry);
     } else {
-      ev.list[off.y + rs] = ev.stage[slot];
+      flag_error(st, kErrQueueCapacity);
     }
   }
+  if (A.rb.bins) {
+    const uint32_t rank = bin_rank(A.rb.bins, bin);
+    if (bin != kInvalid) A.rb.at[dst] = make_uint2(bin, rank);
+  }
+  if (side) place_side(A, slot, off.y + rs);
 }
 
 __global__ void k_advance(RunState* st, uint32_t by) {
@@ -301,15 +461,16 @@ void photon_emit(const PhotonArgs& a, cudaStream_t s) {
   if (nb == 0) return;
   k_photon_emit<<<nb, kBlock, 0, s>>>(a); note_launch();
   k_queue_scan<<<1, 1024, 0, s>>>(a.st, a.qb.tile_counts, a.qb.tile_offsets, 0, 1, a.photons_per_launch, 0,
-                                  a.ps.capacity); note_launch();
-  k_queue_scatter<0><<<nb, kBlock, 0, s>>>(a.st, a.qb, 0, 1, a.photons_per_launch, a.ps, EventBufs{}); note_launch();
+                                  a.ps.capacity, JobScan{}); note_launch();
+  k_queue_scatter<<<nb, kBlock, 0, s>>>(a, 0u, 1, a.photons_per_launch); note_launch();
 }
 
 void photon_bounce(const PhotonArgs& a, uint32_t parity, cudaStream_t s) {
   const uint32_t nb = blocks_for(a.qb.capacity);
   k_photon_bounce<<<nb, kBlock, top_smem(a.scene), s>>>(a, parity); note_launch();
-  k_queue_scan<<<1, 1024, 0, s>>>(a.st, a.qb.tile_counts, a.qb.tile_offsets, parity, 0, 0, 0, a.ps.capacity); note_launch();
-  k_queue_scatter<0><<<nb, kBlock, 0, s>>>(a.st, a.qb, parity, 0, 0, a.ps, EventBufs{}); note_launch();
+  k_queue_scan<<<1, 1024, 0, s>>>(a.st, a.qb.tile_counts, a.qb.tile_offsets, parity, 0, 0, 0, a.ps.capacity,
+                                  JobScan{}); note_launch();
+  k_queue_scatter<<<nb, kBlock, 0, s>>>(a, parity, 0, 0u); note_launch();
 }
 
 // ------------------------------------------------------------ photon grid
@@ -864,14 +1025,8 @@ __global__ void __launch_bounds__(kBlock) k_cg_lit(FrameArgs A, uint32_t round) 
       }
     }
     if (kSort) {
-      // one atomic per bin present in the warp: a view that looks at one
-      // spot puts most of its records into few bins
-      const unsigned peers = __match_any_sync(0xffffffffu, bin);
-      const int leader = __ffs(peers) - 1;
-      uint32_t base = 0;
-      if (lane == leader && bin != kInvalid) base = atomicAdd(&A.bins[bin], (uint32_t)__popc(peers));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (i < n) A.rec_bin[i] = make_uint2(bin, base + __popc(peers & ((1u << lane) - 1u)));
+      const uint32_t rank = bin_rank(A.bins, bin);
+      if (i < n) A.rec_bin[i] = make_uint2(bin, rank);
     } else {
       const unsigned lit = __ballot_sync(0xffffffffu, bin != kInvalid);
       uint32_t base = 0;
@@ -881,48 +1036,6 @@ __global__ void __launch_bounds__(kBlock) k_cg_lit(FrameArgs A, uint32_t round) 
     }
   }
   warp_count(&A.st->gather_queries, queries);
-}
-
-// Counts -> offsets: every block scans its kBlock * kBinItems bins and takes
-// its range of the order with one atomic.
-constexpr int kBinItems = 8;
-__global__ void __launch_bounds__(kBlock) k_bin_offsets(uint32_t* __restrict__ bins, uint32_t* __restrict__ next) {
-  __shared__ uint32_t s_warp[kBlock / 32];
-  __shared__ uint32_t s_base;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint4* p = reinterpret_cast<uint4*>(bins) + ((size_t)blockIdx.x * kBlock + threadIdx.x) * (kBinItems / 4);
-  uint4 v[kBinItems / 4];
-  uint32_t sum = 0;
-#pragma unroll
-  for (int k = 0; k < kBinItems / 4; ++k) {
-    v[k] = p[k];
-    sum += v[k].x + v[k].y + v[k].z + v[k].w;
-  }
-  uint32_t x = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) s_warp[wid] = x;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < kBlock / 32; ++w) {
-      const uint32_t c = s_warp[w];
-      s_warp[w] = t;
-      t += c;
-    }
-    s_base = t ? atomicAdd(next, t) : 0u;
-  }
-  __syncthreads();
-  uint32_t run = s_base + s_warp[wid] + x - sum;
-#pragma unroll
-  for (int k = 0; k < kBinItems / 4; ++k) {
-    const uint4 c = v[k];
-    p[k] = make_uint4(run, run + c.x, run + c.x + c.y, run + c.x + c.y + c.z);
-    run += c.x + c.y + c.z + c.w;
-  }
 }
 
 __global__ void __launch_bounds__(kBlock) k_cg_order(FrameArgs A, uint32_t round) {
@@ -1353,94 +1466,24 @@ __global__ void k_adj_raygen(AdjointArgs A, uint32_t npaths) {
   A.pend.c[path] = make_uint4(kInvalid, kInvalid, 0u, 0u);
 }
 
-// Queue start of every job after a compaction: exclusive scan of the
-// survivor counts, which are cleared for the bounce after next.
-__global__ void __launch_bounds__(kMaxJobsPerBatch) k_job_scan(AdjointArgs A, uint32_t parity) {
-  __shared__ uint32_t s_w[32];
-  uint32_t* cnt = A.job_count + (size_t)(parity ^ 1u) * kMaxJobsPerBatch;
-  uint32_t* start = A.job_start + (size_t)(parity ^ 1u) * kMaxJobsPerBatch;
-  const uint32_t j = threadIdx.x;
-  const int lane = j & 31, wid = j >> 5;
-  const uint32_t c = j < A.njobs ? cnt[j] : 0u;
-  uint32_t x = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) s_w[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    uint32_t w = s_w[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += y;
-    }
-    s_w[lane] = w;
-  }
-  __syncthreads();
-  start[j] = (wid > 0 ? s_w[wid - 1] : 0u) + x - c;
-  cnt[j] = 0u;
-}
-
-// Sort key of a queued ray: direction octant (3 bits) over the Morton code
-// of its origin on a 512^3 lattice over the photon grid's box (27 bits).
-__device__ __forceinline__ uint32_t spread9(uint32_t v) {
-  v &= 0x1FFu;
-  v = (v | (v << 16)) & 0x030000FFu;
-  v = (v | (v << 8)) & 0x0300F00Fu;
-  v = (v | (v << 4)) & 0x030C30C3u;
-  v = (v | (v << 2)) & 0x09249249u;
-  return v;
-}
-
-// Sort key of a ray: (direction octant, 27-bit Morton code of the origin in
-// its scene's grid box); with several scenes, (scene, octant, 24-bit Morton
-// code), so that the rays of one scene stay together.
-__global__ void k_adj_keys(AdjointArgs A, uint32_t parity) {
-  const uint32_t t = blockIdx.x * kBlock + threadIdx.x;
-  if (t >= A.st->active[parity]) return;
-  const RayRec ry = A.qb.q[parity][t];
-  const uint32_t sid = A.cams[A.jobs[__float_as_uint(ry.d.w) >> 8].cam].scene;
-  const GridView& G = A.scenes.s[sid].grid;
-  uint32_t q[3];
-  const float o[3] = {ry.o.x, ry.o.y, ry.o.z}, lo[3] = {G.origin.x, G.origin.y, G.origin.z},
-              ext[3] = {G.cell.x * G.res[0], G.cell.y * G.res[1], G.cell.z * G.res[2]};
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const float f = (o[k] - lo[k]) / fmaxf(ext[k], 1e-30f) * 512.0f;
-    q[k] = (uint32_t)fminf(fmaxf(f, 0.0f), 511.0f);
-  }
-  const uint32_t oct = (ry.d.x < 0.f ? 1u : 0u) | (ry.d.y < 0.f ? 2u : 0u) | (ry.d.z < 0.f ? 4u : 0u);
-  const uint32_t morton = (spread9(q[0]) << 2) | (spread9(q[1]) << 1) | spread9(q[2]);
-  A.sort_keys[t] = A.scenes.n > 1 ? (sid << 27) | (oct << 24) | (morton >> 3) : (oct << 27) | morton;
-  A.perm[t] = t;
-}
-
-// Per 256-slot tile of the input queue: survivors and events, for the
-// slot-ordered compaction.
-__global__ void k_adj_tile_counts(AdjointArgs A, uint32_t parity) {
-  const uint32_t n_in = A.st->active[parity];
-  if ((uint64_t)blockIdx.x * kBlock >= n_in) return;
-  const uint32_t slot = blockIdx.x * kBlock + threadIdx.x;
-  const uint8_t f = slot < n_in ? A.qb.flags[slot] : 0;
-  const uint32_t ca = __syncthreads_count(f & 1), ce = __syncthreads_count(f & 2);
-  if (threadIdx.x == 0) A.qb.tile_counts[blockIdx.x] = make_uint2(ca, ce);
-}
-
 // intersectScene of the adjoint bounce (AdjointKernels.cpp:87-386 traces
 // with it) in three steps: k_adj_mesh, k_adj_walk, and k_adj_bounce reading
 // their records.  Step 1: the mesh pass of every ray, one thread per ray in
-// the order of the bounce: the closest mesh hit, and the surfel walk's
-// record with its limit (the mesh distance plus intersect_scene's margin)
-// when the ray enters the surfel cloud's box before the mesh hit.
-__global__ void k_adj_mesh(AdjointArgs A, uint32_t parity, int sorted) {
+// slot order: the closest mesh hit, and the surfel walk's record with its
+// limit (the mesh distance plus intersect_scene's margin) when the ray
+// enters the surfel cloud's box before the mesh hit, at the ray's place in
+// the walk's order (its 32 B are one sector wherever they land, while the
+// ray and its hit record are read and written in a row).
+__global__ void k_adj_mesh(AdjointArgs A, uint32_t parity) {
   const uint32_t n_in = A.st->active[parity];
-  const uint32_t t = blockIdx.x * kBlock + threadIdx.x;
-  if (t == 0) A.st->walk_next = 0u;
-  if (t >= n_in) return;
-  const uint32_t slot = sorted ? A.perm[t] : t;
+  const uint32_t slot = blockIdx.x * kBlock + threadIdx.x;
+  if (slot == 0) A.st->walk_next = 0u;
+  if (slot >= n_in) return;
+  uint32_t t = slot;
+  if (A.rb.bins) {
+    const uint2 at = A.rb.at[slot];
+    t = __ldg(&A.rb.bins[at.x]) + at.y;
+  }
   const float4 rd = A.qb.q[parity][slot].d;
   const uint32_t sid = A.cams[A.jobs[__float_as_uint(rd.w) >> 8].cam].scene;
   const SceneView& S = A.scenes.s[sid];
@@ -1681,6 +1724,9 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
     if (alive && (threadIdx.x & 31) == __ffs(peers) - 1)
       atomicAdd(&A.job_count[(size_t)(parity ^ 1u) * kMaxJobsPerBatch + job], (uint32_t)__popc(peers));
   }
+  // the tile's survivors and events, for the slot-ordered compaction
+  const uint32_t ca = __syncthreads_count(alive), ce = __syncthreads_count(has_ev);
+  if (threadIdx.x == 0) A.qb.tile_counts[blockIdx.x] = make_uint2(ca, ce);
   block_count3(&A.st->adjoint_segments, slot < n_in ? 1u : 0u, nullptr, 0u, nullptr, 0u);
 }
 
@@ -2125,16 +2171,15 @@ void adjoint_raygen(const AdjointArgs& a, uint32_t npaths, cudaStream_t s) {
 }
 
 // One bounce of every job of the batch; npaths bounds the live queue.
-void adjoint_bounce(const AdjointArgs& a, uint32_t bounce, uint32_t npaths, cudaStream_t s) {
+void adjoint_bounce(AdjointArgs a, uint32_t bounce, bool last, uint32_t npaths, cudaStream_t s) {
   const uint32_t nb = blocks_for(npaths);
   if (nb == 0) return;
   const uint32_t parity = bounce & 1u;
+  const RayBins rb = a.rb;
   // the first bounce traces camera rays in pixel order, already coherent
-  const int sorted = bounce > 0 && a.perm && npaths <= a.sort_capacity;
-  if (sorted) {
-    k_adj_keys<<<nb, kBlock, 0, s>>>(a, parity); note_launch();
-    radix_sort_pairs(a.sort_keys, a.perm, a.sort_keys_tmp, a.perm_tmp, &a.st->active[parity], npaths, 30,
-                     a.sort_temp, s);
+  if (bounce == 0) a.rb.bins = nullptr;
+  if (a.rb.bins) {
+    k_bin_offsets<<<(1u << rb.log2) / (kBlock * kBinItems), kBlock, 0, s>>>(rb.bins, &a.st->ray_next); note_launch();
   }
   int dev = 0, sms = 148, per_sm = 1;
   cudaGetDevice(&dev);
@@ -2143,7 +2188,7 @@ void adjoint_bounce(const AdjointArgs& a, uint32_t bounce, uint32_t npaths, cuda
   const int wt = a.walk_block == 64 || a.walk_block == 128 ? (int)a.walk_block : kBlock;
   const size_t smem = top_smem(a.scenes, wt);
   if (a.timer) a.timer->begin(kTimeAdjBounce, s);
-  k_adj_mesh<<<nb, kBlock, 0, s>>>(a, parity, sorted); note_launch();
+  k_adj_mesh<<<nb, kBlock, 0, s>>>(a, parity); note_launch();
   // the walk's persistent grid: every SM filled once, no more blocks than rays need
   if (multi) {
     if (wt == 64) launch_walk(k_adj_walk<true, 64>, 64, a, parity, smem, nb, s);
@@ -2156,10 +2201,13 @@ void adjoint_bounce(const AdjointArgs& a, uint32_t bounce, uint32_t npaths, cuda
   }
   k_adj_bounce<<<nb, kBlock, 0, s>>>(a, parity, bounce); note_launch();
   if (a.timer) a.timer->end(s);
-  k_adj_tile_counts<<<nb, kBlock, 0, s>>>(a, parity); note_launch();
-  k_queue_scan<<<1, 1024, 0, s>>>(a.st, a.qb.tile_counts, a.qb.tile_offsets, parity, 0, 0, 1, 0); note_launch();
-  k_job_scan<<<1, kMaxJobsPerBatch, 0, s>>>(a, parity); note_launch();
-  k_queue_scatter<1><<<nb, kBlock, 0, s>>>(a.st, a.qb, parity, 0, 0, PhotonStore{}, a.ev); note_launch();
+  a.rb = rb;
+  if (last) a.rb.bins = nullptr;
+  if (a.rb.bins) cudaMemsetAsync(rb.bins, 0, sizeof(uint32_t) << rb.log2, s);
+  const size_t next = (size_t)(parity ^ 1u) * kMaxJobsPerBatch;
+  k_queue_scan<<<2, 1024, 0, s>>>(a.st, a.qb.tile_counts, a.qb.tile_offsets, parity, 0, 0, 1, 0,
+                                  JobScan{a.job_count + next, a.job_start + next, a.njobs}); note_launch();
+  k_queue_scatter<<<nb, kBlock, 0, s>>>(a, parity, 0, 0u); note_launch();
   // a warp per tile of 32 events: a grid that fills every SM once
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_transport, kBlock, 0);
   if (a.timer) a.timer->begin(kTimeTransport, s);
