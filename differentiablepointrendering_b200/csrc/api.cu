@@ -440,8 +440,11 @@ void alloc_photon_store(pale_handle* h, uint64_t cap) {
   h->photon_cap = cap;
   const size_t pc = (size_t)cap;
   h->ph_a.alloc(pc); h->ph_b.alloc(pc); h->ph_c.alloc(pc);
-  h->g_pa.alloc(pc); h->g_pb.alloc(pc); h->g_pc.alloc(pc);
-  h->g_cell_id.alloc(pc); h->g_sorted.alloc(pc); h->g_keys.alloc(2 * pc); h->g_vals_tmp.alloc(pc);
+  // the grid's copy and its sort's keys also hold the photon passes' trace
+  // buffers (hits, walk records, bins): the passes are over when it is built
+  const size_t pl = h->st.photons_per_launch;
+  h->g_pa.alloc(std::max(pc, 3 * pl)); h->g_pb.alloc(std::max(pc, 2 * pl)); h->g_pc.alloc(pc);
+  h->g_cell_id.alloc(pc); h->g_sorted.alloc(pc); h->g_keys.alloc(2 * std::max(pc, pl)); h->g_vals_tmp.alloc(pc);
   h->g_sort_temp.alloc(radix_temp_words((uint32_t)pc));
 }
 
@@ -926,9 +929,13 @@ void trace_photon_map(pale_handle* h) {
   P.q_reflect = st.q_reflect;
   P.q_transmit = st.q_transmit;
   if (st.photons_per_launch > h->qcap) throw ArgError("photons per launch exceed the queue capacity");
+  P.tr = TraceBufs{h->g_pa.p, h->g_pb.p, st.walk_block};
+  const int bins = ray_bins_log2(st.photons_per_launch);
+  if (bins) h->ray_bins.ensure((size_t)1 << bins);
+  P.rb = RayBins{bins ? h->ray_bins.p : nullptr, reinterpret_cast<uint2*>(h->g_keys.p), bins};
   for (uint32_t pass = 0; pass < st.forward_passes; ++pass) {
     photon_emit(P, s);
-    for (uint32_t b = 0; b < st.max_bounces; ++b) photon_bounce(P, b & 1u, s);
+    for (uint32_t b = 0; b < st.max_bounces; ++b) photon_bounce(P, b & 1u, b + 1 == st.max_bounces, s);
   }
   GridBufs G{};
   G.cell_id = h->g_cell_id.p;
@@ -1343,9 +1350,7 @@ void adjoint_views(const std::vector<pale_handle*>& scenes, const std::vector<Vi
   A.light0_valid = h->n_lights > 0;
   A.light0_area = h->light0_area;
   A.timer = &h->timer;
-  A.hits = h->adj_hits.p;
-  A.walkq = h->adj_walkq.p;
-  A.walk_block = st.walk_block;
+  A.tr = TraceBufs{h->adj_hits.p, h->adj_walkq.p, st.walk_block};
   // jobs in the reference's order (view-major, then pass), packed into
   // batches of at most adj_cap paths and kMaxJobsPerBatch jobs
   const std::vector<uint32_t> slots = seed_slots(scenes, views);

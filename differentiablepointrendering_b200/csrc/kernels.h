@@ -129,6 +129,19 @@ struct RayBins {
   int log2;
 };
 
+// Per queue slot, 3 float4: the closest mesh hit (position and distance,
+// +inf on a miss; alpha, instance bits, primitive bits) and the surfel
+// walk's result (surfel bits, distance, 1 on a hit), which the mesh pass
+// sets to no hit.  Per position t of the walk's order (slot order, or for
+// the bounces after the first the order of RayBins), the walk's record, 2 float4: (origin, walk limit or -1 when
+// the ray does not enter the surfel cloud's box) (unit direction, slot
+// bits).
+struct TraceBufs {
+  float4* hits;
+  float4* walkq;
+  uint32_t walk_block;     // threads per block of the persistent walk (host side)
+};
+
 struct PhotonStore {
   float4* a;              // deposit order: position, power.r
   float4* b;              // incoming direction, power.g
@@ -383,6 +396,7 @@ struct PhotonArgs {
   const uint32_t* seeds;
   QueueBufs qb;
   RayBins rb;
+  TraceBufs tr;
   PhotonStore ps;
   uint32_t photons_per_launch;
   float inv_emitted;
@@ -428,20 +442,11 @@ struct AdjointArgs {
   uint32_t light0_valid;
   float light0_area;
   KernelTimer* timer;      // host side, may be null
-  // Per queue slot, 3 float4: the closest mesh hit (position and distance,
-  // +inf on a miss; alpha, instance bits, primitive bits) and the surfel
-  // walk's result (surfel bits, distance, 1 on a hit), which the mesh pass
-  // sets to no hit.  Per position t of the walk's order (slot order, or for
-  // the bounces after the first the order of RayBins), the walk's record, 2 float4: (origin, walk limit or -1 when
-  // the ray does not enter the surfel cloud's box) (unit direction, slot
-  // bits).
-  float4* hits;
-  float4* walkq;
-  uint32_t walk_block;     // threads per block of the persistent walks (host side)
+  TraceBufs tr;
 };
 
 void photon_emit(const PhotonArgs& a, cudaStream_t s);
-void photon_bounce(const PhotonArgs& a, uint32_t parity, cudaStream_t s);
+void photon_bounce(PhotonArgs a, uint32_t parity, bool last, cudaStream_t s);
 void grid_build(const SceneView& sv, RunState* st, const PhotonStore& ps, const GridBufs& g, uint32_t cells,
                 int key_bits, cudaStream_t s);
 // The camera gather of the views `views` (host copy of a.cams; every view

@@ -318,6 +318,180 @@ __global__ void k_advance(RunState* st, uint32_t by) {
   if (threadIdx.x == 0 && blockIdx.x == 0) st->seed_cursor += by;
 }
 
+// ---------------------------------------------------------- traced bounces
+// A traced bounce (photons, adjoint) is intersect_scene in three steps: the
+// mesh pass (mesh_step, a thread per ray in slot order), the persistent
+// surfel walk (k_ray_walk) and the shading kernel, which reads the two
+// records with closest_hit.
+
+// Step 1: the closest mesh hit of the ray at `slot`, and the surfel walk's
+// record with its limit (the mesh distance plus intersect_scene's margin)
+// when the ray enters the surfel cloud's box before the mesh hit, at the
+// ray's place in the walk's order (its 32 B are one sector wherever they
+// land, while the ray and its hit record are read and written in a row).
+__device__ __forceinline__ void mesh_step(const SceneView& S, V3 o, V3 d, uint32_t slot, uint32_t sid,
+                                          const RayBins& rb, const TraceBufs& tr) {
+  uint32_t t = slot;
+  if (rb.bins) {
+    const uint2 at = rb.at[slot];
+    t = __ldg(&rb.bins[at.x]) + at.y;
+  }
+  const V3 invw = safe_inv(d);
+  float best;
+  const Hit h = intersect_meshes(S, o, d, invw, best);
+  float limit = -1.0f;
+  if (S.has_pc && S.node_count > 0 &&
+      entered(slab_entry(o, invw, S.pc_lo.x, S.pc_lo.y, S.pc_lo.z, S.pc_hi.x, S.pc_hi.y, S.pc_hi.z, best), best))
+    limit = best < 3.0e38f ? best * 1.00001f + 1e-6f : __int_as_float(0x7f800000);
+  tr.hits[3 * (size_t)slot] = make_float4(h.pos.x, h.pos.y, h.pos.z, best);
+  tr.hits[3 * (size_t)slot + 1] = make_float4(h.alpha, __int_as_float(h.inst), __uint_as_float(h.prim), 0.0f);
+  tr.hits[3 * (size_t)slot + 2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const V3 dd = normalize(d);
+  // the slot, in a call of several scenes (an adjoint's, of at most 2^24
+  // rays) with the scene in the top bits
+  tr.walkq[2 * (size_t)t] = make_float4(o.x, o.y, o.z, limit);
+  tr.walkq[2 * (size_t)t + 1] = make_float4(dd.x, dd.y, dd.z, __uint_as_float(slot | (sid << 24)));
+}
+
+// The hit of the ray (o, d) at `slot`: the walk's surfel when its world
+// distance is below the mesh hit's, else the mesh hit.
+__device__ __forceinline__ Hit closest_hit(const SceneView& S, const TraceBufs& tr, uint32_t slot, V3 o, V3 d) {
+  Hit h;
+  const float4 ha = tr.hits[3 * (size_t)slot], hb = tr.hits[3 * (size_t)slot + 1];
+  const float4 wr = tr.hits[3 * (size_t)slot + 2];
+  h.pos = xyz(ha);
+  h.inst = __float_as_int(hb.y);
+  h.prim = __float_as_uint(hb.z);
+  h.alpha = hb.x;
+  h.t = h.inst >= 0 ? ha.w : 3.402823466e+38f;
+  if (wr.z != 0.0f) {
+    const uint32_t prim = __float_as_uint(wr.x);
+    V3 x;
+    float a;
+    surfel_eval(S.sf, prim, o, normalize(d), wr.y, x, a);
+    const float tw = dot(x - o, d);
+    if (tw > 0.0f && tw < ha.w) {
+      h.inst = (int)S.mesh.instances;
+      h.t = tw;
+      h.pos = x;
+      h.prim = prim;
+      h.alpha = a;
+    }
+  }
+  return h;
+}
+
+struct WalkArgs {
+  SceneTable scenes;
+  RunState* st;
+  TraceBufs tr;
+};
+
+// The closest-surfel walks (surfel_closest's) of the rays that enter the
+// cloud, on a persistent grid.  Each lane walks one ray at a
+// time; every kRefillSteps node visits the lanes whose walk has ended take
+// the next rays (one atomic per warp on a cursor over the bounce's order,
+// one load of the walk record each), so that a warp's lanes stay busy
+// while walks of very different lengths end.  A walk that finds a surfel
+// ends with one store of it and its distance in the ray's hit record; the
+// hits do not depend on the schedule.
+template <bool kMulti, int kThreads>
+__global__ void __launch_bounds__(kThreads, kWalkMinBlocks * (kBlock / kThreads))
+    k_ray_walk(WalkArgs A, uint32_t parity) {
+  extern __shared__ TravNode s_top[];
+  stage_top_nodes(A.scenes, s_top);
+  const uint32_t n_in = A.st->active[parity];
+  const int lane = threadIdx.x & 31;
+  TravStack stk(s_top, A.scenes.n * A.scenes.staged);
+  ClosestWalk w;
+  TraceCounters ctr{0, 0};
+  uint32_t sid = 0;          // scene of this lane's ray
+  uint32_t cur = kInvalid;   // queue slot of this lane's ray
+  bool more = true;          // uniform in the warp: the cursor has rays left
+  for (;;) {
+    const unsigned need = __ballot_sync(0xffffffffu, cur == kInvalid);
+    if (need && more) {
+      const int leader = __ffs(need) - 1;
+      uint32_t b0 = 0;
+      if (lane == leader) b0 = atomicAdd(&A.st->walk_next, (uint32_t)__popc(need));
+      b0 = __shfl_sync(0xffffffffu, b0, leader);
+      if ((uint64_t)b0 + __popc(need) >= n_in) more = false;
+      if (cur == kInvalid) {
+        const uint32_t t = b0 + __popc(need & ((1u << lane) - 1u));
+        if (t < n_in) {
+          const float4 wa = A.tr.walkq[2 * (size_t)t], wb = A.tr.walkq[2 * (size_t)t + 1];
+          if (wa.w >= 0.0f) {
+            const uint32_t word = __float_as_uint(wb.w);
+            cur = kMulti ? word & 0x00FFFFFFu : word;
+            if (kMulti) sid = word >> 24;
+            w.init(xyz(wa), xyz(wb), 1e-5f, wa.w);
+          }
+        }
+      }
+    }
+    if (!__any_sync(0xffffffffu, cur != kInvalid)) {
+      if (!more) break;
+      continue;
+    }
+    for (int it = 0; it < kRefillSteps; ++it) {
+      if (!__any_sync(0xffffffffu, cur != kInvalid)) break;
+      const uint32_t sc = kMulti ? sid : 0u;
+      if (warp_step(w, cur != kInvalid, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
+          cur == kInvalid)
+        continue;
+      if (w.hit) A.tr.hits[3 * (size_t)cur + 2] = make_float4(__uint_as_float(w.prim), w.best, 1.0f, 0.0f);
+      cur = kInvalid;
+    }
+  }
+  block_count3(&A.st->node_visits, ctr.nodes, &A.st->surfel_tests, ctr.tests, nullptr, 0u);
+}
+
+// Dynamic shared memory of a traversal kernel: the staged top nodes, then
+// PALE_SMEM_STACK stack entries (8 B) per thread of the block.
+static size_t top_smem(const SceneView& s) {
+  return (size_t)s.top_nodes * sizeof(TravNode) + (size_t)PALE_SMEM_STACK * kBlock * sizeof(uint2);
+}
+static size_t top_smem(const SceneTable& t, int threads = kBlock) {
+  return (size_t)t.n * t.staged * sizeof(TravNode) + (size_t)PALE_SMEM_STACK * threads * sizeof(uint2);
+}
+
+// Launch of a persistent walk kernel with the block size `threads` (64,
+// 128 or 256): one resident wave of blocks (occupancy x SMs), at most
+// `limit` blocks of 256-thread equivalents.
+template <typename KernelT, typename Args>
+static void launch_walk(KernelT kernel, int threads, const Args& a, uint32_t arg, size_t smem, uint32_t limit,
+                        cudaStream_t s) {
+  int dev = 0, sms = 148, per_sm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // the staged nodes of a call of several scenes and the shared stack reach
+  // 48 KB, and the kernel's own static shared memory comes on top: allow
+  // the dynamic part past the default limit
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+  const uint64_t grid = std::min<uint64_t>((uint64_t)limit * (kBlock / threads),
+                                           (uint64_t)std::max(1, sms * std::max(1, per_sm)));
+  kernel<<<(uint32_t)std::max<uint64_t>(1, grid), threads, smem, s>>>(a, arg);
+  note_launch();
+}
+
+// The walk of the rays in queue `parity`: a persistent grid, every SM filled
+// once, no more blocks than `rays` rays need.
+static void ray_walk(const WalkArgs& w, uint32_t parity, uint32_t rays, cudaStream_t s) {
+  const int wt = w.tr.walk_block == 64 || w.tr.walk_block == 128 ? (int)w.tr.walk_block : kBlock;
+  const size_t smem = top_smem(w.scenes, wt);
+  const uint32_t nb = blocks_for(rays);
+  if (w.scenes.n > 1) {
+    if (wt == 64) launch_walk(k_ray_walk<true, 64>, 64, w, parity, smem, nb, s);
+    else if (wt == 128) launch_walk(k_ray_walk<true, 128>, 128, w, parity, smem, nb, s);
+    else launch_walk(k_ray_walk<true, 256>, 256, w, parity, smem, nb, s);
+  } else {
+    if (wt == 64) launch_walk(k_ray_walk<false, 64>, 64, w, parity, smem, nb, s);
+    else if (wt == 128) launch_walk(k_ray_walk<false, 128>, 128, w, parity, smem, nb, s);
+    else launch_walk(k_ray_walk<false, 256>, 256, w, parity, smem, nb, s);
+  }
+}
+
 // --------------------------------------------------------------- photons
 // launchRayGenEmitterKernel (PrimalKernels.cpp:13-62).
 __global__ void k_photon_emit(PhotonArgs A) {
@@ -338,15 +512,21 @@ __global__ void k_photon_emit(PhotonArgs A) {
   if (threadIdx.x == 0) A.qb.tile_counts[blockIdx.x] = make_uint2(c, 0u);
 }
 
-// launchIntersectKernel for the photon pass (PrimalKernels.cpp:65-321).
-__global__ void __launch_bounds__(kBlock) k_photon_bounce(PhotonArgs A, uint32_t parity) {
-  extern __shared__ TravNode s_top[];
+// launchIntersectKernel for the photon pass (PrimalKernels.cpp:65-321), as
+// a traced bounce: k_photon_mesh, k_ray_walk, and k_photon_bounce with the
+// shading.
+__global__ void k_photon_mesh(PhotonArgs A, uint32_t parity) {
+  const uint32_t slot = blockIdx.x * kBlock + threadIdx.x;
+  if (slot == 0) A.st->walk_next = 0u;
+  if (slot >= A.st->active[parity]) return;
+  mesh_step(A.scene, xyz(A.qb.q[parity][slot].o), xyz(A.qb.q[parity][slot].d), slot, 0u, A.rb, A.tr);
+}
+
+__global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_photon_bounce(PhotonArgs A, uint32_t parity) {
   const uint32_t n_in = A.st->active[parity];
   if ((uint64_t)blockIdx.x * kBlock >= n_in) return;
-  stage_top_nodes(A.scene, s_top);
   const uint32_t slot = blockIdx.x * kBlock + threadIdx.x;
   bool alive = false, dep = false;
-  TraceCounters ctr{0, 0};
   if (slot < n_in) {
     const SceneView& S = A.scene;
     const uint64_t base = A.seeds[A.st->seed_cursor];
@@ -354,7 +534,7 @@ __global__ void __launch_bounds__(kBlock) k_photon_bounce(PhotonArgs A, uint32_t
     const RayRec ry = A.qb.q[parity][slot];
     const V3 o = xyz(ry.o), d = xyz(ry.d), thr = xyz(ry.t);
     const uint32_t path = __float_as_uint(ry.o.w), bounce = __float_as_uint(ry.d.w) + 1u;
-    Hit h = intersect_scene(S, s_top, o, d, ctr, A.st);
+    const Hit h = closest_hit(S, A.tr, slot, o, d);
     if (h.inst >= 0) {
       V3 no, nd, nt;
       if (h.inst < (int)S.mesh.instances) {
@@ -421,39 +601,18 @@ __global__ void __launch_bounds__(kBlock) k_photon_bounce(PhotonArgs A, uint32_t
     }
     A.qb.flags[slot] = (alive ? 1 : 0) | (dep ? 2 : 0);
   }
-  block_count3(&A.st->photon_segments, slot < n_in ? 1u : 0u, &A.st->node_visits, ctr.nodes, &A.st->surfel_tests,
-               ctr.tests);
+  block_count3(&A.st->photon_segments, slot < n_in ? 1u : 0u, nullptr, 0u, nullptr, 0u);
   uint32_t ca = __syncthreads_count(alive), cd = __syncthreads_count(dep);
   if (threadIdx.x == 0) A.qb.tile_counts[blockIdx.x] = make_uint2(ca, cd);
 }
 
-// Dynamic shared memory of a traversal kernel: the staged top nodes, then
-// PALE_SMEM_STACK stack entries (8 B) per thread of the block.
-static size_t top_smem(const SceneView& s) {
-  return (size_t)s.top_nodes * sizeof(TravNode) + (size_t)PALE_SMEM_STACK * kBlock * sizeof(uint2);
-}
-static size_t top_smem(const SceneTable& t, int threads = kBlock) {
-  return (size_t)t.n * t.staged * sizeof(TravNode) + (size_t)PALE_SMEM_STACK * threads * sizeof(uint2);
+static void zero_bins(const RayBins& rb, cudaStream_t s) {
+  if (rb.bins) cudaMemsetAsync(rb.bins, 0, sizeof(uint32_t) << rb.log2, s);
 }
 
-// Launch of a persistent walk kernel with the block size `threads` (64,
-// 128 or 256): one resident wave of blocks (occupancy x SMs), at most
-// `limit` blocks of 256-thread equivalents.
-template <typename KernelT, typename Args>
-static void launch_walk(KernelT kernel, int threads, const Args& a, uint32_t arg, size_t smem, uint32_t limit,
-                        cudaStream_t s) {
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // the staged nodes of a call of several scenes and the shared stack reach
-  // 48 KB, and the kernel's own static shared memory comes on top: allow
-  // the dynamic part past the default limit
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-  const uint64_t grid = std::min<uint64_t>((uint64_t)limit * (kBlock / threads),
-                                           (uint64_t)std::max(1, sms * std::max(1, per_sm)));
-  kernel<<<(uint32_t)std::max<uint64_t>(1, grid), threads, smem, s>>>(a, arg);
-  note_launch();
+static void offset_bins(const RayBins& rb, RunState* st, cudaStream_t s) {
+  if (!rb.bins) return;
+  k_bin_offsets<<<(1u << rb.log2) / (kBlock * kBinItems), kBlock, 0, s>>>(rb.bins, &st->ray_next); note_launch();
 }
 
 void photon_emit(const PhotonArgs& a, cudaStream_t s) {
@@ -462,14 +621,29 @@ void photon_emit(const PhotonArgs& a, cudaStream_t s) {
   k_photon_emit<<<nb, kBlock, 0, s>>>(a); note_launch();
   k_queue_scan<<<1, 1024, 0, s>>>(a.st, a.qb.tile_counts, a.qb.tile_offsets, 0, 1, a.photons_per_launch, 0,
                                   a.ps.capacity, JobScan{}); note_launch();
+  zero_bins(a.rb, s);
   k_queue_scatter<<<nb, kBlock, 0, s>>>(a, 0u, 1, a.photons_per_launch); note_launch();
 }
 
-void photon_bounce(const PhotonArgs& a, uint32_t parity, cudaStream_t s) {
-  const uint32_t nb = blocks_for(a.qb.capacity);
-  k_photon_bounce<<<nb, kBlock, top_smem(a.scene), s>>>(a, parity); note_launch();
+// One photon bounce; last: none follows in this pass.
+void photon_bounce(PhotonArgs a, uint32_t parity, bool last, cudaStream_t s) {
+  const uint32_t nb = blocks_for(a.photons_per_launch);   // bounds the queue
+  offset_bins(a.rb, a.st, s);
+  k_photon_mesh<<<nb, kBlock, 0, s>>>(a, parity); note_launch();
+  if (a.scene.node_count) {
+    WalkArgs w{};
+    w.scenes.s[0] = a.scene;
+    w.scenes.n = 1;
+    w.scenes.staged = kTopNodes;
+    w.st = a.st;
+    w.tr = a.tr;
+    ray_walk(w, parity, a.photons_per_launch, s);
+  }
+  k_photon_bounce<<<nb, kBlock, 0, s>>>(a, parity); note_launch();
   k_queue_scan<<<1, 1024, 0, s>>>(a.st, a.qb.tile_counts, a.qb.tile_offsets, parity, 0, 0, 0, a.ps.capacity,
                                   JobScan{}); note_launch();
+  if (last) a.rb.bins = nullptr;
+  zero_bins(a.rb, s);
   k_queue_scatter<<<nb, kBlock, 0, s>>>(a, parity, 0, 0u); note_launch();
 }
 
@@ -714,7 +888,7 @@ __global__ void k_cg_mesh(FrameArgs A, uint32_t round) {
 
 // Round step 1b: the K-closest-surfel walks, on a persistent grid whose
 // lanes take the next queue entries every kRefillSteps node visits once
-// their walk has ended (as k_adj_walk does for the adjoint's closest hits).
+// their walk has ended (as k_ray_walk does for closest hits).
 // A walk ends with one store of its hit count and surfels.
 // kMulti: the call renders several scenes (each lane's scene from its walk
 // record); a one-scene call reads the table's first entry, whose fields the
@@ -1467,106 +1641,19 @@ __global__ void k_adj_raygen(AdjointArgs A, uint32_t npaths) {
 }
 
 // intersectScene of the adjoint bounce (AdjointKernels.cpp:87-386 traces
-// with it) in three steps: k_adj_mesh, k_adj_walk, and k_adj_bounce reading
-// their records.  Step 1: the mesh pass of every ray, one thread per ray in
-// slot order: the closest mesh hit, and the surfel walk's record with its
-// limit (the mesh distance plus intersect_scene's margin) when the ray
-// enters the surfel cloud's box before the mesh hit, at the ray's place in
-// the walk's order (its 32 B are one sector wherever they land, while the
-// ray and its hit record are read and written in a row).
+// with it): k_adj_mesh, k_ray_walk, and k_adj_bounce reading their records.
 __global__ void k_adj_mesh(AdjointArgs A, uint32_t parity) {
-  const uint32_t n_in = A.st->active[parity];
   const uint32_t slot = blockIdx.x * kBlock + threadIdx.x;
   if (slot == 0) A.st->walk_next = 0u;
-  if (slot >= n_in) return;
-  uint32_t t = slot;
-  if (A.rb.bins) {
-    const uint2 at = A.rb.at[slot];
-    t = __ldg(&A.rb.bins[at.x]) + at.y;
-  }
+  if (slot >= A.st->active[parity]) return;
   const float4 rd = A.qb.q[parity][slot].d;
   const uint32_t sid = A.cams[A.jobs[__float_as_uint(rd.w) >> 8].cam].scene;
-  const SceneView& S = A.scenes.s[sid];
-  const V3 o = xyz(A.qb.q[parity][slot].o), d = xyz(rd);
-  const V3 invw = safe_inv(d);
-  float best;
-  const Hit h = intersect_meshes(S, o, d, invw, best);
-  float limit = -1.0f;
-  if (S.has_pc && S.node_count > 0 &&
-      entered(slab_entry(o, invw, S.pc_lo.x, S.pc_lo.y, S.pc_lo.z, S.pc_hi.x, S.pc_hi.y, S.pc_hi.z, best), best))
-    limit = best < 3.0e38f ? best * 1.00001f + 1e-6f : __int_as_float(0x7f800000);
-  A.hits[3 * (size_t)slot] = make_float4(h.pos.x, h.pos.y, h.pos.z, best);
-  A.hits[3 * (size_t)slot + 1] = make_float4(h.alpha, __int_as_float(h.inst), __uint_as_float(h.prim), 0.0f);
-  A.hits[3 * (size_t)slot + 2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  const V3 dd = normalize(d);
-  // the slot (below 2^24) with the scene in the top bits
-  A.walkq[2 * (size_t)t] = make_float4(o.x, o.y, o.z, limit);
-  A.walkq[2 * (size_t)t + 1] = make_float4(dd.x, dd.y, dd.z, __uint_as_float(slot | (sid << 24)));
+  mesh_step(A.scenes.s[sid], xyz(A.qb.q[parity][slot].o), xyz(rd), slot, sid, A.rb, A.tr);
 }
 
-// Step 2: the closest-surfel walks (surfel_closest's) of the rays that
-// enter the cloud, on a persistent grid.  Each lane walks one ray at a
-// time; every kRefillSteps node visits the lanes whose walk has ended take
-// the next rays (one atomic per warp on a cursor over the bounce's order,
-// one load of the walk record each), so that a warp's lanes stay busy
-// while walks of very different lengths end.  A walk that finds a surfel
-// ends with one store of it and its distance in the ray's hit record; the
-// hits do not depend on the schedule.
-template <bool kMulti, int kThreads>
-__global__ void __launch_bounds__(kThreads, kWalkMinBlocks * (kBlock / kThreads))
-    k_adj_walk(AdjointArgs A, uint32_t parity) {
-  extern __shared__ TravNode s_top[];
-  stage_top_nodes(A.scenes, s_top);
-  const uint32_t n_in = A.st->active[parity];
-  const int lane = threadIdx.x & 31;
-  TravStack stk(s_top, A.scenes.n * A.scenes.staged);
-  ClosestWalk w;
-  TraceCounters ctr{0, 0};
-  uint32_t sid = 0;          // scene of this lane's ray
-  uint32_t cur = kInvalid;   // queue slot of this lane's ray
-  bool more = true;          // uniform in the warp: the cursor has rays left
-  for (;;) {
-    const unsigned need = __ballot_sync(0xffffffffu, cur == kInvalid);
-    if (need && more) {
-      const int leader = __ffs(need) - 1;
-      uint32_t b0 = 0;
-      if (lane == leader) b0 = atomicAdd(&A.st->walk_next, (uint32_t)__popc(need));
-      b0 = __shfl_sync(0xffffffffu, b0, leader);
-      if ((uint64_t)b0 + __popc(need) >= n_in) more = false;
-      if (cur == kInvalid) {
-        const uint32_t t = b0 + __popc(need & ((1u << lane) - 1u));
-        if (t < n_in) {
-          const float4 wa = A.walkq[2 * (size_t)t], wb = A.walkq[2 * (size_t)t + 1];
-          if (wa.w >= 0.0f) {
-            const uint32_t word = __float_as_uint(wb.w);
-            cur = word & 0x00FFFFFFu;
-            if (kMulti) sid = word >> 24;
-            w.init(xyz(wa), xyz(wb), 1e-5f, wa.w);
-          }
-        }
-      }
-    }
-    if (!__any_sync(0xffffffffu, cur != kInvalid)) {
-      if (!more) break;
-      continue;
-    }
-    for (int it = 0; it < kRefillSteps; ++it) {
-      if (!__any_sync(0xffffffffu, cur != kInvalid)) break;
-      const uint32_t sc = kMulti ? sid : 0u;
-      if (warp_step(w, cur != kInvalid, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
-          cur == kInvalid)
-        continue;
-      if (w.hit) A.hits[3 * (size_t)cur + 2] = make_float4(__uint_as_float(w.prim), w.best, 1.0f, 0.0f);
-      cur = kInvalid;
-    }
-  }
-  block_count3(&A.st->node_visits, ctr.nodes, &A.st->surfel_tests, ctr.tests, nullptr, 0u);
-}
-
-// Step 3, launchAdjointIntersectKernel (AdjointKernels.cpp:87-386) after
-// its intersection, in slot order (every access coalesced; the sorted
-// order only serves the walks).  The hit is intersect_scene's: the walk's
-// surfel when its world distance is below the mesh hit's, else the mesh hit.
+// launchAdjointIntersectKernel (AdjointKernels.cpp:87-386) after its
+// intersection, in slot order (every access coalesced; the bins' order only
+// serves the walks).
 __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointArgs A, uint32_t parity, uint32_t bounce_index) {
   const uint32_t n_in = A.st->active[parity];
   if ((uint64_t)blockIdx.x * kBlock >= n_in) return;
@@ -1577,32 +1664,7 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
     const float4 ro = A.qb.q[parity][slot].o, rd = A.qb.q[parity][slot].d;
     const SceneView& S = A.scenes.s[A.cams[A.jobs[__float_as_uint(rd.w) >> 8].cam].scene];
     const V3 d = xyz(rd);
-    Hit h;
-    {
-      const float4 ha = A.hits[3 * (size_t)slot], hb = A.hits[3 * (size_t)slot + 1];
-      const float4 wr = A.hits[3 * (size_t)slot + 2];
-      h.pos = xyz(ha);
-      h.inst = __float_as_int(hb.y);
-      h.prim = __float_as_uint(hb.z);
-      h.alpha = hb.x;
-      h.t = h.inst >= 0 ? ha.w : 3.402823466e+38f;
-      const float best = ha.w;
-      if (wr.z != 0.0f) {
-        const V3 o = xyz(ro);
-        const uint32_t prim = __float_as_uint(wr.x);
-        V3 x;
-        float a;
-        surfel_eval(S.sf, prim, o, normalize(d), wr.y, x, a);
-        const float tw = dot(x - o, d);
-        if (tw > 0.0f && tw < best) {
-          h.inst = (int)S.mesh.instances;
-          h.t = tw;
-          h.pos = x;
-          h.prim = prim;
-          h.alpha = a;
-        }
-      }
-    }
+    const Hit h = closest_hit(S, A.tr, slot, xyz(ro), d);
     const float4 rt = A.qb.q[parity][slot].t;
     const uint32_t jb = __float_as_uint(rd.w);
     job = jb >> 8;
@@ -2178,32 +2240,18 @@ void adjoint_bounce(AdjointArgs a, uint32_t bounce, bool last, uint32_t npaths, 
   const RayBins rb = a.rb;
   // the first bounce traces camera rays in pixel order, already coherent
   if (bounce == 0) a.rb.bins = nullptr;
-  if (a.rb.bins) {
-    k_bin_offsets<<<(1u << rb.log2) / (kBlock * kBinItems), kBlock, 0, s>>>(rb.bins, &a.st->ray_next); note_launch();
-  }
+  offset_bins(a.rb, a.st, s);
   int dev = 0, sms = 148, per_sm = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const bool multi = a.scenes.n > 1;
-  const int wt = a.walk_block == 64 || a.walk_block == 128 ? (int)a.walk_block : kBlock;
-  const size_t smem = top_smem(a.scenes, wt);
   if (a.timer) a.timer->begin(kTimeAdjBounce, s);
   k_adj_mesh<<<nb, kBlock, 0, s>>>(a, parity); note_launch();
-  // the walk's persistent grid: every SM filled once, no more blocks than rays need
-  if (multi) {
-    if (wt == 64) launch_walk(k_adj_walk<true, 64>, 64, a, parity, smem, nb, s);
-    else if (wt == 128) launch_walk(k_adj_walk<true, 128>, 128, a, parity, smem, nb, s);
-    else launch_walk(k_adj_walk<true, 256>, 256, a, parity, smem, nb, s);
-  } else {
-    if (wt == 64) launch_walk(k_adj_walk<false, 64>, 64, a, parity, smem, nb, s);
-    else if (wt == 128) launch_walk(k_adj_walk<false, 128>, 128, a, parity, smem, nb, s);
-    else launch_walk(k_adj_walk<false, 256>, 256, a, parity, smem, nb, s);
-  }
+  ray_walk(WalkArgs{a.scenes, a.st, a.tr}, parity, npaths, s);
   k_adj_bounce<<<nb, kBlock, 0, s>>>(a, parity, bounce); note_launch();
   if (a.timer) a.timer->end(s);
   a.rb = rb;
   if (last) a.rb.bins = nullptr;
-  if (a.rb.bins) cudaMemsetAsync(rb.bins, 0, sizeof(uint32_t) << rb.log2, s);
+  zero_bins(a.rb, s);
   const size_t next = (size_t)(parity ^ 1u) * kMaxJobsPerBatch;
   k_queue_scan<<<2, 1024, 0, s>>>(a.st, a.qb.tile_counts, a.qb.tile_offsets, parity, 0, 0, 1, 0,
                                   JobScan{a.job_count + next, a.job_start + next, a.njobs}); note_launch();
