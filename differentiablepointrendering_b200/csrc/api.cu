@@ -221,8 +221,9 @@ struct pale_handle {
   DBuf<uint2> tile_counts, tile_offsets;
   DBuf<float4> pend_a, pend_b;
   DBuf<uint4> pend_c;
-  DBuf<EventRec> ev_stage, ev_list;
-  DBuf<float4> adj_hits;   // hit record per adjoint queue slot (3 float4)
+  DBuf<EventRec> ev_list;
+  DBuf<float4> ev_ext;     // with gradients = all (2 float4 per event)
+  DBuf<float4> adj_hits;   // hit record per adjoint queue slot (2 float4)
   DBuf<float4> adj_walkq;  // walk record per sorted position (2 float4)
   // adjoint batches
   uint32_t adj_cap = 0;
@@ -443,7 +444,7 @@ void alloc_photon_store(pale_handle* h, uint64_t cap) {
   // the grid's copy and its sort's keys also hold the photon passes' trace
   // buffers (hits, walk records, bins): the passes are over when it is built
   const size_t pl = h->st.photons_per_launch;
-  h->g_pa.alloc(std::max(pc, 3 * pl)); h->g_pb.alloc(std::max(pc, 2 * pl)); h->g_pc.alloc(pc);
+  h->g_pa.alloc(std::max(pc, 2 * pl)); h->g_pb.alloc(std::max(pc, 2 * pl)); h->g_pc.alloc(pc);
   h->g_cell_id.alloc(pc); h->g_sorted.alloc(pc); h->g_keys.alloc(2 * std::max(pc, pl)); h->g_vals_tmp.alloc(pc);
   h->g_sort_temp.alloc(radix_temp_words((uint32_t)pc));
 }
@@ -484,8 +485,9 @@ void size_wavefronts(pale_handle* h, uint64_t all_pix, uint32_t max_pix) {
     h->ray_bins.ensure((size_t)1 << ray_bins_log2(h->adj_cap));
     size_queues(h, qa);
     h->pend_a.alloc(qa); h->pend_b.alloc(qa); h->pend_c.alloc(qa);
-    h->ev_stage.alloc(qa); h->ev_list.alloc(qa);
-    h->adj_hits.alloc(3 * qa);
+    h->ev_list.alloc(qa);
+    if (st.gradients == PALE_GRADIENTS_ALL) h->ev_ext.alloc(2 * qa);
+    h->adj_hits.alloc(2 * qa);
     h->adj_walkq.alloc(2 * qa);
   }
   const uint64_t want = all_pix * std::max<uint32_t>(1u, st.gather_passes);
@@ -1336,7 +1338,7 @@ void adjoint_views(const std::vector<pale_handle*>& scenes, const std::vector<Vi
   A.qb = QueueBufs{{h->q0.p, h->q1.p}, h->qstage.p, h->qflags.p, h->tile_counts.p, h->tile_offsets.p,
                    std::max(h->qcap, h->adj_cap)};
   A.pend = PendingBufs{h->pend_a.p, h->pend_b.p, h->pend_c.p};
-  A.ev = EventBufs{h->ev_stage.p, h->ev_list.p};
+  A.ev = EventBufs{h->ev_list.p, h->ev_ext.p};
   A.dldi = d_dldi;
   A.all_grads = st.gradients == PALE_GRADIENTS_ALL;
   A.debug_opacity = d_dbg;

@@ -129,13 +129,13 @@ struct RayBins {
   int log2;
 };
 
-// Per queue slot, 3 float4: the closest mesh hit (position and distance,
-// +inf on a miss; alpha, instance bits, primitive bits) and the surfel
-// walk's result (surfel bits, distance, 1 on a hit), which the mesh pass
-// sets to no hit.  Per position t of the walk's order (slot order, or for
-// the bounces after the first the order of RayBins), the walk's record, 2 float4: (origin, walk limit or -1 when
-// the ray does not enter the surfel cloud's box) (unit direction, slot
-// bits).
+// Per queue slot, 2 float4: the closest mesh hit (position and distance,
+// +inf on a miss) and (instance bits, primitive bits, the surfel walk's
+// surfel bits and its distance, -1 for no hit, as the mesh pass sets it).
+// Per position t of the walk's order (slot order, or for the bounces after
+// the first the order of RayBins), the walk's record, 2 float4: (origin,
+// walk limit or -1 when the ray does not enter the surfel cloud's box)
+// (unit direction, slot bits).
 struct TraceBufs {
   float4* hits;
   float4* walkq;
@@ -182,13 +182,14 @@ struct EventRec {
   float4 b;   // gather normal, endpoint pdf or endpoint cosine
   float4 c;   // path throughput, -
   uint4 d;    // kind, target surfel, material, pixel
-  float4 e;   // hit position on the target surfel (its alpha term's point), -
-  float4 f;   // unit ray direction at that hit, -
 };
 
+// The events of a bounce, in no particular order.  ext, only with gradients
+// of every group, holds per event the hit position on its target surfel (its
+// alpha term's point) and the unit ray direction at that hit.
 struct EventBufs {
-  EventRec* stage;        // per slot
-  EventRec* list;         // compacted, slot order
+  EventRec* list;
+  float4* ext;
 };
 
 // The scenes of one render call.  A call renders views (a camera of a scene

@@ -163,8 +163,8 @@ int ray_bins_log2(uint32_t rays) {
 }
 
 // ---------------------------------------------------------- compaction
-// One block: exclusive scan of the per-tile (alive, deposit/event) counts
-// of `n_in` slots; updates queue length, deposit/event bases and seeds.  The
+// One block: exclusive scan of the per-tile (alive, deposit) counts of
+// `n_in` slots; updates queue length, deposit bases and seeds.  The
 // adjoint launches a second block for its jobs: the queue start of every job
 // after the compaction is the exclusive scan of the survivor counts, which
 // are cleared for the bounce after next.
@@ -202,7 +202,7 @@ __device__ __forceinline__ void scan_jobs(const JobScan& js, uint32_t* s_w) {
 
 static_assert(kMaxJobsPerBatch == 1024, "scan_jobs: a thread per job");
 __global__ void __launch_bounds__(1024) k_queue_scan(RunState* st, const uint2* __restrict__ counts, uint2* __restrict__ offsets,
-                             uint32_t parity, int emission, uint32_t emission_n, int events, uint64_t photon_cap,
+                             uint32_t parity, int emission, uint32_t emission_n, int adjoint, uint64_t photon_cap,
                              JobScan jobs) {
   __shared__ uint32_t s_wx[32], s_wy[32];
   __shared__ uint32_t s_carry[2];
@@ -249,9 +249,7 @@ __global__ void __launch_bounds__(1024) k_queue_scan(RunState* st, const uint2* 
   }
   if (threadIdx.x == 0) {
     st->active[emission ? 0u : (parity ^ 1u)] = s_carry[0];
-    if (events) {
-      st->event_count = s_carry[1];
-    } else {
+    if (!adjoint) {
       st->photon_base = st->photon_attempts;
       st->photon_attempts += s_carry[1];
       if ((uint64_t)st->photon_base + s_carry[1] > photon_cap) atomicOr(&st->error, kErrPhotonCapacity);
@@ -261,7 +259,7 @@ __global__ void __launch_bounds__(1024) k_queue_scan(RunState* st, const uint2* 
   }
 }
 
-// Compacts staged rays (and deposits or events) of the `n_in` input slots,
+// Compacts staged rays (and photon deposits) of the `n_in` input slots,
 // and takes the rays into their bins for the next bounce's walk.
 __device__ __forceinline__ void place_side(const PhotonArgs& A, uint32_t slot, uint32_t rank) {
   const uint64_t dst = (uint64_t)A.st->photon_base + rank;
@@ -271,11 +269,9 @@ __device__ __forceinline__ void place_side(const PhotonArgs& A, uint32_t slot, u
     A.ps.c[dst] = A.ps.sc[slot];
   }
 }
-__device__ __forceinline__ void place_side(const AdjointArgs& A, uint32_t slot, uint32_t rank) {
-  A.ev.list[rank] = A.ev.stage[slot];
-}
+__device__ __forceinline__ void place_side(const AdjointArgs&, uint32_t, uint32_t) {}
 
-template <class Args>   // PhotonArgs (deposits), AdjointArgs (events)
+template <class Args>   // PhotonArgs, AdjointArgs
 __global__ void k_queue_scatter(Args A, uint32_t parity, int emission, uint32_t emission_n) {
   RunState* st = A.st;
   const QueueBufs& qb = A.qb;
@@ -343,9 +339,8 @@ __device__ __forceinline__ void mesh_step(const SceneView& S, V3 o, V3 d, uint32
   if (S.has_pc && S.node_count > 0 &&
       entered(slab_entry(o, invw, S.pc_lo.x, S.pc_lo.y, S.pc_lo.z, S.pc_hi.x, S.pc_hi.y, S.pc_hi.z, best), best))
     limit = best < 3.0e38f ? best * 1.00001f + 1e-6f : __int_as_float(0x7f800000);
-  tr.hits[3 * (size_t)slot] = make_float4(h.pos.x, h.pos.y, h.pos.z, best);
-  tr.hits[3 * (size_t)slot + 1] = make_float4(h.alpha, __int_as_float(h.inst), __uint_as_float(h.prim), 0.0f);
-  tr.hits[3 * (size_t)slot + 2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  tr.hits[2 * (size_t)slot] = make_float4(h.pos.x, h.pos.y, h.pos.z, best);
+  tr.hits[2 * (size_t)slot + 1] = make_float4(__int_as_float(h.inst), __uint_as_float(h.prim), 0.0f, -1.0f);
   const V3 dd = normalize(d);
   // the slot, in a call of several scenes (an adjoint's, of at most 2^24
   // rays) with the scene in the top bits
@@ -357,18 +352,17 @@ __device__ __forceinline__ void mesh_step(const SceneView& S, V3 o, V3 d, uint32
 // distance is below the mesh hit's, else the mesh hit.
 __device__ __forceinline__ Hit closest_hit(const SceneView& S, const TraceBufs& tr, uint32_t slot, V3 o, V3 d) {
   Hit h;
-  const float4 ha = tr.hits[3 * (size_t)slot], hb = tr.hits[3 * (size_t)slot + 1];
-  const float4 wr = tr.hits[3 * (size_t)slot + 2];
+  const float4 ha = tr.hits[2 * (size_t)slot], hb = tr.hits[2 * (size_t)slot + 1];
   h.pos = xyz(ha);
-  h.inst = __float_as_int(hb.y);
-  h.prim = __float_as_uint(hb.z);
-  h.alpha = hb.x;
+  h.inst = __float_as_int(hb.x);
+  h.prim = __float_as_uint(hb.y);
+  h.alpha = 0.0f;
   h.t = h.inst >= 0 ? ha.w : 3.402823466e+38f;
-  if (wr.z != 0.0f) {
-    const uint32_t prim = __float_as_uint(wr.x);
+  if (hb.w >= 0.0f) {
+    const uint32_t prim = __float_as_uint(hb.z);
     V3 x;
     float a;
-    surfel_eval(S.sf, prim, o, normalize(d), wr.y, x, a);
+    surfel_eval(S.sf, prim, o, normalize(d), hb.w, x, a);
     const float tw = dot(x - o, d);
     if (tw > 0.0f && tw < ha.w) {
       h.inst = (int)S.mesh.instances;
@@ -439,7 +433,8 @@ __global__ void __launch_bounds__(kThreads, kWalkMinBlocks * (kBlock / kThreads)
       if (warp_step(w, cur != kInvalid, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
           cur == kInvalid)
         continue;
-      if (w.hit) A.tr.hits[3 * (size_t)cur + 2] = make_float4(__uint_as_float(w.prim), w.best, 1.0f, 0.0f);
+      if (w.hit)
+        *reinterpret_cast<float2*>(&A.tr.hits[2 * (size_t)cur + 1].z) = make_float2(__uint_as_float(w.prim), w.best);
       cur = kInvalid;
     }
   }
@@ -1644,7 +1639,7 @@ __global__ void k_adj_raygen(AdjointArgs A, uint32_t npaths) {
 // with it): k_adj_mesh, k_ray_walk, and k_adj_bounce reading their records.
 __global__ void k_adj_mesh(AdjointArgs A, uint32_t parity) {
   const uint32_t slot = blockIdx.x * kBlock + threadIdx.x;
-  if (slot == 0) A.st->walk_next = 0u;
+  if (slot == 0) A.st->walk_next = A.st->event_count = 0u;
   if (slot >= A.st->active[parity]) return;
   const float4 rd = A.qb.q[parity][slot].d;
   const uint32_t sid = A.cams[A.jobs[__float_as_uint(rd.w) >> 8].cam].scene;
@@ -1658,13 +1653,17 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
   const uint32_t n_in = A.st->active[parity];
   if ((uint64_t)blockIdx.x * kBlock >= n_in) return;
   const uint32_t slot = blockIdx.x * kBlock + threadIdx.x;
-  bool alive = false, has_ev = false;
+  bool alive = false, has_ev = false, put_ev = false;
+  EventRec ev;
+  V3 ev_x;
   uint32_t job = kInvalid;
+  V3 ev_d;
   if (slot < n_in) {
     const float4 ro = A.qb.q[parity][slot].o, rd = A.qb.q[parity][slot].d;
     const SceneView& S = A.scenes.s[A.cams[A.jobs[__float_as_uint(rd.w) >> 8].cam].scene];
     const V3 d = xyz(rd);
     const Hit h = closest_hit(S, A.tr, slot, xyz(ro), d);
+    ev_d = normalize(d);
     const float4 rt = A.qb.q[parity][slot].t;
     const uint32_t jb = __float_as_uint(rd.w);
     job = jb >> 8;
@@ -1691,7 +1690,6 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
       const float4 pa = A.pend.a[path], pb = A.pend.b[path];
       const uint4 pc = A.pend.c[path];
       const uint32_t pkind = __float_as_uint(pb.w);
-      EventRec ev;
       if ((pkind == kKindReflect && !is_mesh) || pkind == kKindNull) {
         const bool refl = pkind == kKindReflect;
         V3 pthr = scale(xyz(pb), refl ? A.q_reflect : A.q_null);
@@ -1705,14 +1703,14 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
         ev.d = make_uint4(pkind, refl ? h.prim : pc.x, mat, pc.z);
         // the target surfel's hit: the endpoint (reflect) or the pending
         // null surfel, on the same line (a null continuation keeps d)
-        ev.e = f4(refl ? h.pos : xyz(pa), 0.f);
-        ev.f = f4(normalize(d), 0.f);
+        ev_x = refl ? h.pos : xyz(pa);
         has_ev = true;
-        A.pend.b[path] = make_float4(0.f, 0.f, 0.f, __uint_as_float(kKindNone));
-        A.pend.a[path] = make_float4(0.f, 0.f, 0.f, 0.f);
-        A.pend.c[path] = make_uint4(kInvalid, pc.y, 0u, 0u);
+        // a null event that ends on a surfel has no material and adds
+        // nothing: only the debug image shows it
+        put_ev = refl || mat != kInvalid || A.debug_opacity;
       }
       V3 no, nd, nt;
+      bool kept = false;   // this hit is the path's next pending interaction
       if (is_mesh) {
         const float4 mat = __ldg(&S.mesh.materials[__ldg(&S.mesh.material[h.inst])]);
         no = h.pos + scale(nrm, 1e-6f);
@@ -1721,6 +1719,7 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
         alive = russian_roulette(r, bounce, nt, A.rr_start);
         if (alive) {
           V3 pt = mul(thr, xyz(mat));
+          kept = true;
           A.pend.a[path] = f4(h.pos, 0.0f);
           A.pend.b[path] = f4(pt, __uint_as_float(kKindReflect));
           A.pend.c[path] = make_uint4(kInvalid, (uint32_t)h.inst, pixel, 0u);
@@ -1736,6 +1735,7 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
           nt = scale(thr, w);
           alive = russian_roulette(r, bounce, nt, A.rr_start);
           if (alive) {
+            kept = true;
             A.pend.a[path] = f4(h.pos, h.alpha);
             A.pend.b[path] = f4(divs(thr, A.q_null), __uint_as_float(kKindNull));
             A.pend.c[path] = make_uint4(h.prim, kInvalid, pixel, 0u);
@@ -1755,9 +1755,8 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
             ev.b = f4(on, 0.f);
             ev.c = f4(divs(thr, A.q_reflect), __uint_as_float(job));
             ev.d = make_uint4(kKindProjection, h.prim, kInvalid, pixel);
-            ev.e = f4(h.pos, 0.f);
-            ev.f = f4(normalize(d), 0.f);
-            has_ev = true;
+            ev_x = h.pos;
+            has_ev = put_ev = true;
           }
         } else if (u < A.q_null + A.q_reflect + A.q_transmit) {
           float alpha = h.alpha * opacity;
@@ -1772,12 +1771,27 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
           alive = russian_roulette(r, bounce, nt, A.rr_start);
         }
       }
+      if (has_ev && !kept) A.pend.b[path] = make_float4(0.f, 0.f, 0.f, __uint_as_float(kKindNone));
       // a view's rays end after its own number of bounces
       if (alive && bounce >= A.cams[A.jobs[job].cam].depth) alive = false;
       if (alive) A.qb.stage[slot] = make_ray(no, nd, nt, path, bounce | (job << 8), pixel);
-      if (has_ev) A.ev.stage[slot] = ev;
     }
-    A.qb.flags[slot] = (alive ? 1 : 0) | (has_ev ? 2 : 0);
+    A.qb.flags[slot] = alive ? 1 : 0;
+  }
+  {
+    // the events, one atomic per warp
+    const unsigned pm = __ballot_sync(0xffffffffu, put_ev);
+    uint32_t base = 0;
+    if (pm && (threadIdx.x & 31) == 0) base = atomicAdd(&A.st->event_count, (uint32_t)__popc(pm));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (put_ev) {
+      const uint32_t e = base + __popc(pm & ((1u << (threadIdx.x & 31)) - 1u));
+      A.ev.list[e] = ev;
+      if (A.all_grads) {
+        A.ev.ext[2 * (size_t)e] = f4(ev_x, 0.f);
+        A.ev.ext[2 * (size_t)e + 1] = f4(ev_d, 0.f);
+      }
+    }
   }
   {
     // survivors per job, one atomic per job present in the warp
@@ -1786,10 +1800,10 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_adj_bounce(AdjointA
     if (alive && (threadIdx.x & 31) == __ffs(peers) - 1)
       atomicAdd(&A.job_count[(size_t)(parity ^ 1u) * kMaxJobsPerBatch + job], (uint32_t)__popc(peers));
   }
-  // the tile's survivors and events, for the slot-ordered compaction
-  const uint32_t ca = __syncthreads_count(alive), ce = __syncthreads_count(has_ev);
-  if (threadIdx.x == 0) A.qb.tile_counts[blockIdx.x] = make_uint2(ca, ce);
-  block_count3(&A.st->adjoint_segments, slot < n_in ? 1u : 0u, nullptr, 0u, nullptr, 0u);
+  // the tile's survivors, for the slot-ordered compaction
+  const uint32_t ca = __syncthreads_count(alive);
+  if (threadIdx.x == 0) A.qb.tile_counts[blockIdx.x] = make_uint2(ca, 0u);
+  block_count3(&A.st->adjoint_segments, slot < n_in ? 1u : 0u, &A.st->gradient_events, has_ev ? 1u : 0u, nullptr, 0u);
 }
 
 // Derivatives of eta * alpha_geom for the hit at x on surfel k along the
@@ -2065,7 +2079,7 @@ __global__ void __launch_bounds__(kBlock, kTransportMinBlocks) k_transport(Adjoi
   while (per > 2u && count < per * warps) per >>= 1;
   const uint32_t tiles = (count + per - 1u) / per;
   const int nterms = A.all_grads ? kTransportTerms + 1 : 1;
-  uint32_t events = 0, queries = 0, scanned = 0;
+  uint32_t queries = 0, scanned = 0;
   for (uint32_t tile = blockIdx.x * (kBlock / 32) + wid; tile < tiles; tile += warps) {
     const uint32_t e = tile * per + lane;
     const bool valid = lane < per && e < count;
@@ -2115,7 +2129,6 @@ __global__ void __launch_bounds__(kBlock, kTransportMinBlocks) k_transport(Adjoi
     V3 dalb = v3(0.f, 0.f, 0.f);
     uint32_t target = kInvalid;
     if (valid) {
-      ++events;
       const V3 thr = xyz(src->c);
       if (kind == kKindProjection) {
         target = ev.d.y;
@@ -2168,7 +2181,7 @@ __global__ void __launch_bounds__(kBlock, kTransportMinBlocks) k_transport(Adjoi
     val[0][lane] = g;
     if (A.all_grads) {
       AlphaGrad ag{};
-      if (target != kInvalid && W != 0.f) ag = alpha_grad(S.sf, target, xyz(src->e), xyz(src->f));
+      if (target != kInvalid && W != 0.f) ag = alpha_grad(S.sf, target, xyz(A.ev.ext[2 * (size_t)e]), xyz(A.ev.ext[2 * (size_t)e + 1]));
       const bool w0 = target != kInvalid && W != 0.f;
       val[1][lane] = w0 ? W * ag.beta : 0.f;
       val[2][lane] = w0 ? W * ag.pos.x : 0.f;
@@ -2223,7 +2236,6 @@ __global__ void __launch_bounds__(kBlock, kTransportMinBlocks) k_transport(Adjoi
     }
     __syncwarp();
   }
-  warp_count(&A.st->gradient_events, events);
   warp_count(&A.st->gather_queries, queries);
   warp_count(&A.st->photons_scanned, scanned);
 }
