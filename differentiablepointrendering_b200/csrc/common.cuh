@@ -133,8 +133,11 @@ static_assert(sizeof(BvhNode) == 64, "node layout");
 // Traversal copy of a node: the two child boxes in half precision rounded
 // outwards (lower corners down, upper corners up, so a box only grows and
 // no hit is lost) and the two child words, 32 B against BvhNode's 64 B.
-//   q0 = halves (c0.lo.x c0.lo.y) (c0.lo.z c0.hi.x) (c0.hi.y c0.hi.z) (c1.lo.x c1.lo.y)
-//   q1 = halves (c1.lo.z c1.hi.x) (c1.hi.y c1.hi.z), word0, word1
+//   q0 = halves (c0.lo.x c0.lo.y) (c0.hi.x c0.hi.y) (c1.lo.x c1.lo.y) (c1.hi.x c1.hi.y)
+//   q1 = halves (c0.lo.z c1.lo.z) (c0.hi.z c1.hi.z), word0, word1
+// Low and high corners sit in like words, so that one byte permutation picks
+// the near (or far) x and y plane of a child, or the z planes of both, and a
+// packed multiply-add takes a word's two planes to distances.
 struct BvhNodeH {
   uint4 q0;
   uint4 q1;
@@ -145,14 +148,7 @@ static_assert(sizeof(BvhNodeH) == 32, "node layout");
 #define PALE_SMEM_STACK 8
 #endif
 
-#ifndef PALE_HALF_NODES
-#define PALE_HALF_NODES 1
-#endif
-#if PALE_HALF_NODES
 using TravNode = BvhNodeH;
-#else
-using TravNode = BvhNode;
-#endif
 
 // Surfel arrays in BVH (leaf) order.
 struct SurfelView {

@@ -111,14 +111,29 @@ __device__ __forceinline__ void surfel_eval(const SurfelView& sf, uint32_t i, V3
   x_out = x;
 }
 
-#if PALE_HALF_NODES
-__device__ __forceinline__ float2 half_pair(uint32_t v) {
-  return __half22float2(*reinterpret_cast<const __half2*>(&v));
+// Two floats in a 64-bit register, for the packed multiply-add.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long half2_to_float2(uint32_t v) {
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
+  return pack2(f.x, f.y);
 }
 
 __device__ __forceinline__ void load_node(const SceneView& S, const TravNode* __restrict__ smem_top, uint32_t idx,
-                                          float4& a, float4& b, float4& c, uint4& w) {
-  uint4 q0, q1;
+                                          uint4& q0, uint4& q1) {
   if (idx < S.top_nodes) {
     q0 = smem_top[idx].q0;
     q1 = smem_top[idx].q1;
@@ -127,25 +142,46 @@ __device__ __forceinline__ void load_node(const SceneView& S, const TravNode* __
     q0 = __ldg(&nd->q0);
     q1 = __ldg(&nd->q1);
   }
-  const float2 p0 = half_pair(q0.x), p1 = half_pair(q0.y), p2 = half_pair(q0.z), p3 = half_pair(q0.w);
-  const float2 p4 = half_pair(q1.x), p5 = half_pair(q1.y);
-  a = make_float4(p0.x, p0.y, p1.x, p1.y);
-  b = make_float4(p2.x, p2.y, p3.x, p3.y);
-  c = make_float4(p4.x, p4.y, p5.x, p5.y);
-  w = make_uint4(q1.z, q1.w, 0u, 0u);
 }
-#else
-__device__ __forceinline__ void load_node(const SceneView& S, const TravNode* __restrict__ smem_top, uint32_t idx,
-                                          float4& a, float4& b, float4& c, uint4& w) {
-  if (idx < S.top_nodes) {
-    const BvhNode& nd = smem_top[idx];
-    a = nd.a; b = nd.b; c = nd.c; w = nd.d;
-  } else {
-    const BvhNode* nd = S.nodes + idx;
-    a = __ldg(&nd->a); b = __ldg(&nd->b); c = __ldg(&nd->c); w = __ldg(&nd->d);
+
+// A ray as the node test wants it: 1/d and -o/d by planes (x, y) and (z,
+// z), and the byte permutations that pick the near and far planes by the
+// signs of the direction.
+struct NodeRay {
+  unsigned long long inv_xy, inv_zz, no_xy, no_zz;
+  uint32_t near_xy, near_z;
+  __device__ __forceinline__ void set(V3 o, V3 inv) {
+    inv_xy = pack2(inv.x, inv.y);
+    inv_zz = pack2(inv.z, inv.z);
+    no_xy = pack2(-(o.x * inv.x), -(o.y * inv.y));
+    no_zz = pack2(-(o.z * inv.z), -(o.z * inv.z));
+    near_xy = (inv.x < 0.0f ? 0x54u : 0x10u) | (inv.y < 0.0f ? 0x7600u : 0x3200u);
+    near_z = inv.z < 0.0f ? 0x7654u : 0x3210u;
   }
+};
+
+// The slab tests of a node's two child boxes: e0, e1 the entry distances,
+// and whether a box is entered no farther than `best` (slab_entry and
+// entered(): in front of the origin, not past the current closest hit).  A
+// plane's distance is one multiply-add, plane / d - o / d: against (plane -
+// o) / d its rounding moves the origin by up to an ulp, far less than the
+// boxes exceed their surfels (1e-4 of the scale and 1e-3 of the normal, and
+// the rounding to half precision), so no hit is lost.
+__device__ __forceinline__ void node_test(const NodeRay& r, const uint4& q0, const uint4& q1, float best, float& e0,
+                                          float& e1, bool& h0, bool& h1) {
+  const uint32_t far_xy = r.near_xy ^ 0x4444u, far_z = r.near_z ^ 0x4444u;
+  const float2 n0 = unpack2(fma2(half2_to_float2(__byte_perm(q0.x, q0.y, r.near_xy)), r.inv_xy, r.no_xy));
+  const float2 f0 = unpack2(fma2(half2_to_float2(__byte_perm(q0.x, q0.y, far_xy)), r.inv_xy, r.no_xy));
+  const float2 n1 = unpack2(fma2(half2_to_float2(__byte_perm(q0.z, q0.w, r.near_xy)), r.inv_xy, r.no_xy));
+  const float2 f1 = unpack2(fma2(half2_to_float2(__byte_perm(q0.z, q0.w, far_xy)), r.inv_xy, r.no_xy));
+  const float2 nz = unpack2(fma2(half2_to_float2(__byte_perm(q1.x, q1.y, r.near_z)), r.inv_zz, r.no_zz));
+  const float2 fz = unpack2(fma2(half2_to_float2(__byte_perm(q1.x, q1.y, far_z)), r.inv_zz, r.no_zz));
+  e0 = fmaxf(fmaxf(n0.x, n0.y), nz.x);
+  e1 = fmaxf(fmaxf(n1.x, n1.y), nz.y);
+  const float x0 = fminf(fminf(fminf(f0.x, f0.y), fz.x), best), x1 = fminf(fminf(fminf(f1.x, f1.y), fz.y), best);
+  h0 = fmaxf(e0, 0.0f) <= x0;
+  h1 = fmaxf(e1, 0.0f) <= x1;
 }
-#endif
 
 // The traversal stack of one thread: its first PALE_SMEM_STACK entries in
 // shared memory after the staged top nodes (entry k of thread t at
@@ -204,18 +240,17 @@ struct TravStack {
 // test (a closest hit, or the K closest hits).
 template <class Leaf>
 struct WalkBase {
-  V3 o, d, inv;
+  V3 o, d;
+  NodeRay ray;
   float tmin;
   uint32_t node, visit;
-  float node_t;
   int sp;
   __device__ __forceinline__ void start(V3 o_, V3 d_, float tmin_) {
     o = o_;
     d = d_;
-    inv = safe_inv(d_);
+    ray.set(o_, safe_inv(d_));
     tmin = tmin_;
     node = 0;        // the root, an inner node
-    node_t = 0.0f;
     visit = 0;
     sp = 0;
   }
@@ -229,7 +264,6 @@ struct WalkBase {
       stk.get(sp, sn, st_t);
       if (st_t <= best) {
         node = sn;
-        node_t = st_t;
         return true;
       }
     }
@@ -239,15 +273,14 @@ struct WalkBase {
                                        TraceCounters& ctr, RunState* st) {
     Leaf& self = *static_cast<Leaf*>(this);
     if (at_leaf()) {
-      if (node_t <= self.best) {
-        const uint32_t f0 = node & 0x0FFFFFFFu, cnt = ((node >> 28) & 7u) + 1u;
-        if (f0 + cnt > S.sf.count) {
-          flag_error(st, kErrBounds);
-        } else {
-          for (uint32_t j = 0; j < cnt; ++j) {
-            ctr.tests++;
-            self.test(S.sf, f0 + j);
-          }
+      // (its box was entered within `best`, which only this test changes)
+      const uint32_t f0 = node & 0x0FFFFFFFu, cnt = ((node >> 28) & 7u) + 1u;
+      if (f0 + cnt > S.sf.count) {
+        flag_error(st, kErrBounds);
+      } else {
+        for (uint32_t j = 0; j < cnt; ++j) {
+          ctr.tests++;
+          self.test(S.sf, f0 + j);
         }
       }
       return pop(stk, self.best);
@@ -259,39 +292,30 @@ struct WalkBase {
       return false;
     }
     ++visit;
-    float4 a, b, c;
-    uint4 w;
-    load_node(S, smem_top, node, a, b, c, w);
+    uint4 q0, q1;
+    load_node(S, smem_top, node, q0, q1);
     ctr.nodes++;
-    const float best = self.best;
-    const float e0 =
-        w.x == kEmptyChild ? __int_as_float(0x7f800000) : slab_entry(o, inv, a.x, a.y, a.z, a.w, b.x, b.y, best);
-    const float e1 =
-        w.y == kEmptyChild ? __int_as_float(0x7f800000) : slab_entry(o, inv, b.z, b.w, c.x, c.y, c.z, c.w, best);
-    const bool h0 = entered(e0, best), h1 = entered(e1, best);
+    float e0, e1;
+    bool h0, h1;
+    node_test(ray, q0, q1, self.best, e0, e1, h0, h1);
+    h0 = h0 && q1.z != kEmptyChild;
+    h1 = h1 && q1.w != kEmptyChild;
     if (h0 && h1) {
       const bool first0 = e0 <= e1;
       if (sp < kStackDepth) {
-        stk.push(sp, first0 ? w.y : w.x, first0 ? e1 : e0);
+        stk.push(sp, first0 ? q1.w : q1.z, first0 ? e1 : e0);
         ++sp;
       } else {
         flag_error(st, kErrStackOverflow);
       }
-      node = first0 ? w.x : w.y;
-      node_t = first0 ? e0 : e1;
+      node = first0 ? q1.z : q1.w;
       return true;
     }
-    if (h0) {
-      node = w.x;
-      node_t = e0;
+    if (h0 || h1) {
+      node = h0 ? q1.z : q1.w;
       return true;
     }
-    if (h1) {
-      node = w.y;
-      node_t = e1;
-      return true;
-    }
-    return pop(stk, best);
+    return pop(stk, self.best);
   }
 };
 

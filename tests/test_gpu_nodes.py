@@ -1,0 +1,47 @@
+"""Closest hits through the traversal nodes against the oracle for the
+directions and positions where the node test could lose one: axis-parallel
+and nearly parallel rays, negative zeros, every octant, clouds away from the
+origin and of another size, few surfels and leaves of several."""
+import numpy as np
+import pytest
+
+from differentiablepointrendering_b200.pale import Renderer
+from differentiablepointrendering_b200.scene import make_box_scene, make_surfels
+from oracle_lib import OracleRenderer
+
+pytestmark = pytest.mark.gpu
+
+
+def _rays(n, rng, centre, size):
+    o = centre + size * rng.uniform(-0.6, 0.6, (n, 3))
+    d = rng.normal(size=(n, 3))
+    k = n // 2
+    a = rng.integers(0, 3, k)
+    d[:k] = rng.choice([0.0, -0.0, 1e-7, -1e-7, 1e-5], (k, 3))
+    d[np.arange(k), a] = rng.choice([-1.0, 1.0], k)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    return o.astype(np.float32), d.astype(np.float32)
+
+
+@pytest.mark.parametrize("leaf", [1, 4])
+@pytest.mark.parametrize("n,centre,size", [(1, 0.0, 1.0), (3, 0.0, 1.0), (4000, 0.0, 1.0), (4000, 7.3, 1.0),
+                                           (4000, -20.0, 40.0)])
+def test_closest_hits_match_oracle(gpu, n, centre, size, leaf):
+    pts = make_surfels(n, 3)
+    pts["position"] = (centre + size * pts["position"]).astype(np.float32)
+    pts["scale"] = (np.float32(2.0 * size) * pts["scale"]).astype(np.float32)
+    scene = make_box_scene(n, points=pts)
+    st = {"photons": 64, "bounces": 1, "gather_radius": 0.2 * max(size, 1.0), "leaf_size": leaf}
+    g, o = Renderer.from_scene(scene, st), OracleRenderer(scene, st)
+    rays = _rays(20000, np.random.default_rng(1), centre, size)
+    gi, gp, gt, ga, gx = g.trace_rays(*rays)
+    oi, op, ot, oa, ox = o.trace_rays(*rays)
+    go, oo = g.get_point_order(), o.get_point_order()
+    g.close()
+    o.close()
+    assert np.mean(gi == oi) >= 0.9995
+    s = (gi == oi) & (gi == scene.instance_mesh.shape[0])
+    assert s.any() or n < 10
+    assert not s.any() or np.mean(go[gp[s]] == oo[op[s]]) >= 0.9995
+    hit = (gi == oi) & (gi >= 0)
+    np.testing.assert_allclose(gt[hit], ot[hit], rtol=1e-5, atol=1e-6 * max(1.0, size))
