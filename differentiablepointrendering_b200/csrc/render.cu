@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kThreads, kWalkMinBlocks * (kBlock / kThreads)
     for (int it = 0; it < kRefillSteps; ++it) {
       if (!__any_sync(0xffffffffu, cur != kInvalid)) break;
       const uint32_t sc = kMulti ? sid : 0u;
-      if (warp_step(w, cur != kInvalid, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
+      if (warp_step<kLeafBatch>(w, cur != kInvalid, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
           cur == kInvalid)
         continue;
       if (w.hit)
@@ -938,7 +938,7 @@ __global__ void __launch_bounds__(kThreads, kRoundMinBlocks * (kBlock / kThreads
     for (int it = 0; it < kRefillSteps; ++it) {
       if (!__any_sync(0xffffffffu, cur != kInvalid)) break;
       const uint32_t sc = kMulti ? sid : 0u;
-      if (warp_step(w, cur != kInvalid, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
+      if (warp_step<kKHitLeafBatch>(w, cur != kInvalid, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
           cur == kInvalid)
         continue;
       uint32_t rw[kKHitWords];

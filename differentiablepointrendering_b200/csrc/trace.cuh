@@ -449,18 +449,18 @@ struct KHitWalkS : WalkBase<KHitWalkS<K>> {
 };
 
 // One step of a persistent walk loop for the lanes of a warp: the lanes
-// whose walk stands at a leaf step together once at least kLeafBatch of
+// whose walk stands at a leaf step together once at least kBatch of
 // them (or all of the walking lanes) do, the other times the lanes at inner
 // nodes step.  Returns for this lane whether its walk goes on (a lane that
 // sat out the step keeps walking).  Every lane of the warp calls it.
-template <class W>
+template <int kBatch, class W>
 __device__ __forceinline__ bool warp_step(W& w, bool walking, const SceneView& S,
                                           const TravNode* __restrict__ smem_top, TravStack& stk, TraceCounters& ctr,
                                           RunState* st) {
   const bool lf = walking && w.at_leaf();
   const unsigned ml = __ballot_sync(0xffffffffu, lf);
   const unsigned ma = __ballot_sync(0xffffffffu, walking);
-  const bool leaf_phase = ml != 0u && (ml == ma || __popc(ml) >= kLeafBatch);
+  const bool leaf_phase = ml != 0u && (ml == ma || __popc(ml) >= kBatch);
   if (walking && lf == leaf_phase) return w.step(S, smem_top, stk, ctr, st);
   return walking;
 }
