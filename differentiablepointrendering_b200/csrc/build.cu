@@ -51,14 +51,23 @@ __device__ __forceinline__ uint32_t block_exclusive_sum(uint32_t v, uint32_t* s_
   return warp_prefix + x - v;
 }
 
-__global__ void k_scan_reduce(const uint32_t* __restrict__ in, uint32_t n, uint32_t* __restrict__ partial) {
+// Items [i, i + 4) of `in`, zero from n on; i is a multiple of 4 and `in`
+// 16-byte aligned (the callers' arrays are whole allocations or multiples of
+// 256 words into one).
+__device__ __forceinline__ uint4 load_items(const uint32_t* __restrict__ in, size_t i, uint32_t n) {
+  if (i + 4 <= n) return __ldg(reinterpret_cast<const uint4*>(in + i));
+  return make_uint4(i < n ? in[i] : 0u, i + 1 < n ? in[i + 1] : 0u, i + 2 < n ? in[i + 2] : 0u, 0u);
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* __restrict__ in, uint32_t n,
+                                                              uint32_t* __restrict__ partial) {
   __shared__ uint32_t s_warp[32];
   const size_t base = (size_t)blockIdx.x * kScanTile;
   uint32_t sum = 0;
-#pragma unroll 4
-  for (int k = 0; k < kScanItems; ++k) {
-    size_t i = base + (size_t)k * kScanThreads + threadIdx.x;
-    if (i < n) sum += in[i];
+#pragma unroll
+  for (int k = 0; k < kScanItems / 4; ++k) {
+    const uint4 v = load_items(in, base + 4 * ((size_t)k * kScanThreads + threadIdx.x), n);
+    sum += v.x + v.y + v.z + v.w;
   }
   uint32_t total;
   block_exclusive_sum(sum, s_warp, total);
@@ -69,17 +78,17 @@ __global__ void k_scan_reduce(const uint32_t* __restrict__ in, uint32_t n, uint3
 __global__ void __launch_bounds__(1024) k_scan_partials(uint32_t* __restrict__ partial, uint32_t nb,
                                                         uint32_t* __restrict__ total_out) {
   __shared__ uint32_t s_warp[32];
-  const int items = 32;
+  const uint32_t items = (nb + 1023u) / 1024u;
   uint32_t sum = 0;
   const uint32_t base = threadIdx.x * items;
-  for (int k = 0; k < items; ++k) {
+  for (uint32_t k = 0; k < items; ++k) {
     uint32_t i = base + k;
     sum += i < nb ? partial[i] : 0u;
   }
   uint32_t total;
   uint32_t run = block_exclusive_sum(sum, s_warp, total);
   // each thread rewrites only its own consecutive range
-  for (int k = 0; k < items; ++k) {
+  for (uint32_t k = 0; k < items; ++k) {
     uint32_t i = base + k;
     if (i < nb) {
       uint32_t v = partial[i];
@@ -90,18 +99,56 @@ __global__ void __launch_bounds__(1024) k_scan_partials(uint32_t* __restrict__ p
   if (threadIdx.x == 0 && total_out) *total_out = total;
 }
 
-__global__ void k_scan_apply(const uint32_t* __restrict__ in, uint32_t n, const uint32_t* __restrict__ partial,
-                             uint32_t* __restrict__ out) {
-  __shared__ uint32_t s_warp[32];
-  const size_t base = (size_t)blockIdx.x * kScanTile;
-  uint32_t carry = partial[blockIdx.x];
-  for (int k = 0; k < kScanItems; ++k) {
-    size_t i = base + (size_t)k * kScanThreads + threadIdx.x;
-    uint32_t v = i < n ? in[i] : 0u;
-    uint32_t total;
-    uint32_t ex = block_exclusive_sum(v, s_warp, total);
-    if (i < n) out[i] = carry + ex;
-    carry += total;
+// One tile per block: a warp scans 1024 consecutive items, eight rows of 128
+// held in registers (one load latency for all of them), and the warps meet
+// once; a barrier per 256 items, as in a thread-per-item loop, is 96 of them
+// a tile (11 us a launch however little there is to scan, against 3 us).
+// `partial`: the tiles' offsets, or null for a single tile, which then also
+// writes the total.
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __restrict__ in, uint32_t n,
+                                                             const uint32_t* __restrict__ partial,
+                                                             uint32_t* __restrict__ out,
+                                                             uint32_t* __restrict__ total_out) {
+  constexpr int kRows = kScanItems / 4, kWarps = kScanThreads / 32;
+  __shared__ uint32_t s_warp[kWarps];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)wid * (kScanTile / kWarps) + 4 * lane;
+  uint4 v[kRows];
+#pragma unroll
+  for (int k = 0; k < kRows; ++k) v[k] = load_items(in, base + 128 * k, n);
+  uint32_t ex[kRows], run = 0;
+#pragma unroll
+  for (int k = 0; k < kRows; ++k) {
+    const uint32_t sum = v[k].x + v[k].y + v[k].z + v[k].w;
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    ex[k] = run + x - sum;
+    run += __shfl_sync(0xffffffffu, x, 31);
+  }
+  if (lane == 0) s_warp[wid] = run;
+  __syncthreads();
+  uint32_t carry = partial ? partial[blockIdx.x] : 0u, total = carry;
+#pragma unroll
+  for (int w = 0; w < kWarps; ++w) {
+    if (w < wid) carry += s_warp[w];
+    total += s_warp[w];
+  }
+  if (!partial && total_out && threadIdx.x == 0) *total_out = total;
+#pragma unroll
+  for (int k = 0; k < kRows; ++k) {
+    const size_t i = base + 128 * k;
+    const uint32_t a = carry + ex[k], b = a + v[k].x, c = b + v[k].y, d = c + v[k].z;
+    if (i + 4 <= n) {
+      *reinterpret_cast<uint4*>(out + i) = make_uint4(a, b, c, d);
+    } else {
+      if (i < n) out[i] = a;
+      if (i + 1 < n) out[i + 1] = b;
+      if (i + 2 < n) out[i + 2] = c;
+    }
   }
 }
 
@@ -111,9 +158,13 @@ void exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* tem
                     cudaStream_t s) {
   if (n == 0) return;
   uint32_t nb = (n + kScanTile - 1) / kScanTile;
+  if (nb == 1) {
+    k_scan_apply<<<1, kScanThreads, 0, s>>>(in, n, nullptr, out, total); note_launch();
+    return;
+  }
   k_scan_reduce<<<nb, kScanThreads, 0, s>>>(in, n, temp); note_launch();
   k_scan_partials<<<1, 1024, 0, s>>>(temp, nb, total); note_launch();
-  k_scan_apply<<<nb, kScanThreads, 0, s>>>(in, n, temp, out); note_launch();
+  k_scan_apply<<<nb, kScanThreads, 0, s>>>(in, n, temp, out, nullptr); note_launch();
 }
 
 // ------------------------------------------------------------ radix sort
@@ -140,42 +191,55 @@ __global__ void k_radix_hist(const uint32_t* __restrict__ keys, const uint32_t* 
   hist[(size_t)threadIdx.x * tiles + blockIdx.x] = s_cnt[threadIdx.x];
 }
 
-__global__ void k_radix_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-                                const uint32_t* __restrict__ d_n, uint32_t shift, uint32_t tiles,
-                                const uint32_t* __restrict__ offsets, uint32_t* __restrict__ keys_out,
-                                uint32_t* __restrict__ vals_out) {
+// A warp takes 256 consecutive keys of the tile, 32 at a time, and ranks each
+// among its own keys so far (a counter per digit); the warps then meet twice,
+// to turn their counters into places.  (Ranking the block's 256 keys of a
+// round together met four times a round, eight rounds a tile.)
+__global__ void __launch_bounds__(kSortThreads) k_radix_scatter(
+    const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, const uint32_t* __restrict__ d_n,
+    uint32_t shift, uint32_t tiles, const uint32_t* __restrict__ offsets, uint32_t* __restrict__ keys_out,
+    uint32_t* __restrict__ vals_out) {
   constexpr int kWarps = kSortThreads / 32;
-  __shared__ uint32_t s_run[256];
   __shared__ uint32_t s_wcnt[kWarps][256];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t n = *d_n;
-  s_run[threadIdx.x] = offsets[(size_t)threadIdx.x * tiles + blockIdx.x];
-  const size_t base = (size_t)blockIdx.x * kSortTile;
+  if ((size_t)blockIdx.x * kSortTile >= n) return;
+  for (int d = lane; d < 256; d += 32) s_wcnt[wid][d] = 0;
+  __syncwarp();
+  const size_t base = (size_t)blockIdx.x * kSortTile + (size_t)wid * (kSortItems * 32) + lane;
+  uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
+#pragma unroll
   for (int k = 0; k < kSortItems; ++k) {
-    for (int w = 0; w < kWarps; ++w) s_wcnt[w][threadIdx.x] = 0;
-    __syncthreads();
-    size_t i = base + (size_t)k * kSortThreads + threadIdx.x;
-    bool valid = i < n;
-    uint32_t key = valid ? keys_in[i] : 0u;
-    uint32_t val = valid ? vals_in[i] : 0u;
-    uint32_t digit = valid ? ((key >> shift) & 255u) : 256u + (uint32_t)lane;  // unique sentinel per lane
-    unsigned peers = __match_any_sync(0xffffffffu, digit);
-    unsigned lt = (1u << lane) - 1u;
-    uint32_t rank_in_warp = __popc(peers & lt);
-    if (valid && rank_in_warp == 0) s_wcnt[wid][digit] = __popc(peers);
-    __syncthreads();
-    if (valid) {
-      uint32_t before = 0;
-      for (int w = 0; w < wid; ++w) before += s_wcnt[w][digit];
-      uint32_t dst = s_run[digit] + before + rank_in_warp;
-      keys_out[dst] = key;
-      vals_out[dst] = val;
+    const size_t i = base + 32 * k;
+    key[k] = i < n ? keys_in[i] : 0u;
+    val[k] = i < n ? vals_in[i] : 0u;
+  }
+#pragma unroll
+  for (int k = 0; k < kSortItems; ++k) {
+    const bool valid = base + 32 * k < n;
+    const uint32_t digit = valid ? ((key[k] >> shift) & 255u) : 256u + (uint32_t)lane;  // unique sentinel per lane
+    const unsigned peers = __match_any_sync(0xffffffffu, digit);
+    const uint32_t before = valid ? s_wcnt[wid][digit] : 0u;
+    rank[k] = before + __popc(peers & ((1u << lane) - 1u));
+    __syncwarp();
+    if (valid && lane == __ffs(peers) - 1) s_wcnt[wid][digit] = before + __popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  uint32_t run = offsets[(size_t)threadIdx.x * tiles + blockIdx.x];
+  for (int w = 0; w < kWarps; ++w) {
+    const uint32_t c = s_wcnt[w][threadIdx.x];
+    s_wcnt[w][threadIdx.x] = run;
+    run += c;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kSortItems; ++k) {
+    if (base + 32 * k < n) {
+      const uint32_t dst = s_wcnt[wid][(key[k] >> shift) & 255u] + rank[k];
+      keys_out[dst] = key[k];
+      vals_out[dst] = val[k];
     }
-    __syncthreads();
-    uint32_t add = 0;
-    for (int w = 0; w < kWarps; ++w) add += s_wcnt[w][threadIdx.x];
-    s_run[threadIdx.x] += add;
-    __syncthreads();
   }
 }
 
@@ -193,8 +257,8 @@ void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32
   const uint32_t tiles = (n_max + kSortTile - 1) / kSortTile;
   const size_t h = (size_t)tiles * 256;
   uint32_t* hist = temp;
-  uint32_t* offs = temp + h + 1;
-  uint32_t* stemp = offs + h + 1;
+  uint32_t* offs = temp + h;   // (16-byte aligned with temp, for the scan)
+  uint32_t* stemp = offs + h;
   int passes = (bits + 7) / 8;
   uint32_t *ka = keys, *va = vals, *kb = keys_tmp, *vb = vals_tmp;
   for (int p = 0; p < passes; ++p) {
@@ -258,7 +322,7 @@ __global__ void k_collect(PointsDev asset, uint32_t n, PointsDev col, float* __r
 // Min/max of positions and of boxes: per-block partials, then one block.
 __global__ void k_bounds_partial(const float* __restrict__ pos, const float* __restrict__ lo,
                                  const float* __restrict__ hi, uint32_t n, float* __restrict__ part) {
-  __shared__ float s[12][kBlock];
+  __shared__ float s[12][kBlock / 32];
   float acc[12];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -277,23 +341,37 @@ __global__ void k_bounds_partial(const float* __restrict__ pos, const float* __r
     }
   }
 #pragma unroll
-  for (int k = 0; k < 12; ++k) s[k][threadIdx.x] = acc[k];
+  for (int k = 0; k < 12; ++k) {
+    const bool is_min = (k < 3) || (k >= 6 && k < 9);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float y = __shfl_xor_sync(0xffffffffu, acc[k], o);
+      acc[k] = is_min ? fminf(acc[k], y) : fmaxf(acc[k], y);
+    }
+    if ((threadIdx.x & 31) == 0) s[k][threadIdx.x >> 5] = acc[k];
+  }
   __syncthreads();
   if (threadIdx.x < 12) {
     int k = threadIdx.x;
     bool is_min = (k < 3) || (k >= 6 && k < 9);
     float r = s[k][0];
-    for (int t = 1; t < kBlock; ++t) r = is_min ? fminf(r, s[k][t]) : fmaxf(r, s[k][t]);
+    for (int t = 1; t < kBlock / 32; ++t) r = is_min ? fminf(r, s[k][t]) : fmaxf(r, s[k][t]);
     part[12 * blockIdx.x + k] = r;
   }
 }
-__global__ void k_bounds_final(const float* __restrict__ part, uint32_t nb, float* __restrict__ out) {
-  int k = threadIdx.x;
-  if (k >= 12) return;
-  bool is_min = (k < 3) || (k >= 6 && k < 9);
+// A warp per bound.
+__global__ void __launch_bounds__(12 * 32) k_bounds_final(const float* __restrict__ part, uint32_t nb,
+                                                          float* __restrict__ out) {
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool is_min = (k < 3) || (k >= 6 && k < 9);
   float r = part[k];
-  for (uint32_t b = 1; b < nb; ++b) r = is_min ? fminf(r, part[12 * b + k]) : fmaxf(r, part[12 * b + k]);
-  out[k] = r;
+  for (uint32_t b = lane; b < nb; b += 32) r = is_min ? fminf(r, part[12 * b + k]) : fmaxf(r, part[12 * b + k]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float y = __shfl_xor_sync(0xffffffffu, r, o);
+    r = is_min ? fminf(r, y) : fmaxf(r, y);
+  }
+  if (lane == 0) out[k] = r;
 }
 
 // Morton expandBits (Karras 2012).
@@ -467,32 +545,52 @@ __global__ void k_emit_nodes(const uint32_t* __restrict__ order, uint32_t n, con
   nodes[top + x] = nd;
 }
 
-// Breadth-first copy of the first `top` kept nodes into slots [0, top).
-__global__ void k_top_nodes(const uint32_t* __restrict__ rfirst, const uint32_t* __restrict__ rlast, uint32_t n,
-                            uint32_t leaf_size, uint32_t top, BvhNode* __restrict__ nodes) {
-  extern __shared__ uint32_t s_top[];   // [top] source Karras index, [top] map
+// Breadth-first copy of the first `top` kept nodes into slots [0, top): level
+// by level, a thread per node of the level, its kept children placed behind
+// the list by a scan over the level (in the order a queue would take them);
+// the level that fills the list is the last.
+__global__ void __launch_bounds__(kBlock) k_top_nodes(const uint32_t* __restrict__ rfirst,
+                                                      const uint32_t* __restrict__ rlast, uint32_t n,
+                                                      uint32_t leaf_size, uint32_t top, BvhNode* __restrict__ nodes) {
+  extern __shared__ uint32_t s_top[];   // [top] source Karras index, [2 top] slots of its children
+  __shared__ uint32_t s_warp[32];
   uint32_t* src = s_top;
-  __shared__ uint32_t s_count;
-  if (threadIdx.x == 0) {
-    uint32_t cnt = 0, head = 0;
-    if (top > 0) src[cnt++] = 0;
-    while (head < cnt) {
-      uint32_t x = src[head++];
-      BvhNode nd = nodes[top + x];
-      uint32_t ws[2] = {nd.d.x, nd.d.y};
-      for (int c = 0; c < 2; ++c) {
-        uint32_t wd = ws[c];
-        if (wd == kEmptyChild || (wd & kLeafFlag)) continue;
-        uint32_t y = wd - top;
-        if (rlast[y] - rfirst[y] + 1u <= leaf_size) continue;
-        if (cnt >= top) continue;
-        src[cnt++] = y;
-      }
-    }
-    s_count = cnt;
-  }
+  uint32_t* child = s_top + top;
+  for (uint32_t k = threadIdx.x; k < 2 * top; k += blockDim.x) child[k] = kEmptyChild;
+  if (threadIdx.x == 0 && top > 0) src[0] = 0;
   __syncthreads();
-  const uint32_t cnt = s_count;
+  uint32_t first = 0, cnt = top > 0 ? 1u : 0u;   // the level [first, cnt)
+  while (first < cnt && cnt < top) {
+    const uint32_t last = cnt;
+    for (uint32_t b = first; b < last; b += blockDim.x) {
+      const uint32_t k = b + threadIdx.x;
+      uint32_t y[2] = {kEmptyChild, kEmptyChild}, m = 0;
+      if (k < last) {
+        const uint4 d = nodes[top + src[k]].d;
+        const uint32_t ws[2] = {d.x, d.y};
+        for (int c = 0; c < 2; ++c) {
+          if (ws[c] == kEmptyChild || (ws[c] & kLeafFlag)) continue;
+          const uint32_t x = ws[c] - top;
+          if (rlast[x] - rfirst[x] + 1u <= leaf_size) continue;
+          y[c] = x;
+          ++m;
+        }
+      }
+      uint32_t total;
+      uint32_t at = cnt + block_exclusive_sum(m, s_warp, total);
+      for (int c = 0; c < 2; ++c) {
+        if (y[c] == kEmptyChild) continue;
+        if (at < top) {
+          src[at] = y[c];
+          child[2 * k + c] = at;
+        }
+        ++at;
+      }
+      cnt = cnt + total < top ? cnt + total : top;
+      __syncthreads();
+    }
+    first = last;
+  }
   for (uint32_t k = threadIdx.x; k < top; k += blockDim.x) {
     if (k >= cnt) {
       BvhNode z;
@@ -502,16 +600,8 @@ __global__ void k_top_nodes(const uint32_t* __restrict__ rfirst, const uint32_t*
       continue;
     }
     BvhNode nd = nodes[top + src[k]];
-    uint32_t ws[2] = {nd.d.x, nd.d.y};
-    for (int c = 0; c < 2; ++c) {
-      uint32_t wd = ws[c];
-      if (wd == kEmptyChild || (wd & kLeafFlag)) continue;
-      uint32_t y = wd - top;
-      for (uint32_t m = 0; m < cnt; ++m)
-        if (src[m] == y) { ws[c] = m; break; }
-    }
-    nd.d.x = ws[0];
-    nd.d.y = ws[1];
+    if (child[2 * k] != kEmptyChild) nd.d.x = child[2 * k];
+    if (child[2 * k + 1] != kEmptyChild) nd.d.y = child[2 * k + 1];
     nodes[k] = nd;
   }
 }
@@ -583,7 +673,7 @@ void lbvh_build(const LbvhArgs& A, cudaStream_t s) {
   k_collect<<<blocks_for(n), kBlock, 0, s>>>(A.asset, n, A.collected, A.lo, A.hi); note_launch();
   uint32_t nb = blocks_for(n) < 148u * 4u ? blocks_for(n) : 148u * 4u;
   k_bounds_partial<<<nb, kBlock, 0, s>>>(A.collected.position, A.lo, A.hi, n, A.bounds_part); note_launch();
-  k_bounds_final<<<1, 32, 0, s>>>(A.bounds_part, nb, A.bounds); note_launch();
+  k_bounds_final<<<1, 12 * 32, 0, s>>>(A.bounds_part, nb, A.bounds); note_launch();
   k_morton<<<blocks_for(n), kBlock, 0, s>>>(A.collected.position, n, A.bounds, A.codes, A.order); note_launch();
   radix_sort_pairs(A.codes, A.order, A.codes_tmp, A.order_tmp, A.d_n, n, 30, A.sort_temp, s);
   if (n <= A.leaf_size) {
@@ -597,7 +687,7 @@ void lbvh_build(const LbvhArgs& A, cudaStream_t s) {
     k_emit_nodes<<<blocks_for(n - 1), kBlock, 0, s>>>(A.order, n, A.lo, A.hi, A.lc, A.rc, A.rfirst, A.rlast, A.box,
                                                       A.leaf_size, A.top, A.nodes); note_launch();
     if (A.top > 0)
-      k_top_nodes<<<1, kBlock, A.top * sizeof(uint32_t), s>>>(A.rfirst, A.rlast, n, A.leaf_size, A.top, A.nodes); note_launch();
+      k_top_nodes<<<1, kBlock, 3 * A.top * sizeof(uint32_t), s>>>(A.rfirst, A.rlast, n, A.leaf_size, A.top, A.nodes); note_launch();
   }
   k_permute<<<blocks_for(n), kBlock, 0, s>>>(A.collected, A.order, n, A.params); note_launch();
   derive_surfels(A.params, n, A.derived, s);
@@ -767,7 +857,7 @@ extern "C" int pale_build_lbvh_noalloc(const float* d_position, const float* d_t
   k_collect<<<blocks_for(n), kBlock, 0, s>>>(asset, n, col, lo, hi);
   uint32_t nb = blocks_for(n) < 148u * 4u ? blocks_for(n) : 148u * 4u;
   k_bounds_partial<<<nb, kBlock, 0, s>>>(col.position, lo, hi, n, bounds_part);
-  k_bounds_final<<<1, 32, 0, s>>>(bounds_part, nb, bounds);
+  k_bounds_final<<<1, 12 * 32, 0, s>>>(bounds_part, nb, bounds);
   k_morton<<<blocks_for(n), kBlock, 0, s>>>(col.position, n, bounds, d_codes, d_order);
   radix_sort_pairs(d_codes, d_order, codes_tmp, order_tmp, words, n, 30, sort_temp, s);
   if (n <= leaf) {
@@ -778,7 +868,7 @@ extern "C" int pale_build_lbvh_noalloc(const float* d_position, const float* d_t
     cudaMemsetAsync(visits, 0, (size_t)(n - 1) * 4, s);
     k_refit<<<blocks_for(n), kBlock, 0, s>>>(d_order, n, lo, hi, lc, rc, parent, leaf_parent, visits, box);
     k_emit_nodes<<<blocks_for(n - 1), kBlock, 0, s>>>(d_order, n, lo, hi, lc, rc, rfirst, rlast, box, leaf, top, nodes);
-    k_top_nodes<<<1, kBlock, top * sizeof(uint32_t), s>>>(rfirst, rlast, n, leaf, top, nodes);
+    k_top_nodes<<<1, kBlock, 3 * top * sizeof(uint32_t), s>>>(rfirst, rlast, n, leaf, top, nodes);
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) {
