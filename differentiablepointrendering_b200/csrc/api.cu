@@ -276,6 +276,7 @@ struct pale_handle {
   // density control scratch
   DBuf<uint32_t> dc_keys, dc_vals, dc_keys_tmp, dc_vals_tmp, dc_sort_temp, dc_flags, dc_dst, dc_list, dc_word, dc_aux;
   PointsBufs dc_points;
+  DBuf<float> query;          // inputs and outputs of the ray and lookup queries (the largest call's)
   HostStage stage;            // staging of large host copies
   pale_stats stats{};
   uint64_t launches_last = 0;  // kernels launched by the last render call
@@ -1404,27 +1405,54 @@ void backward(pale_handle* h, uint32_t nsel, const uint32_t* idx, const float* d
   adjoint_views({h}, all_passes(h, nsel, idx, h->st.estimator != PALE_ESTIMATOR_GATHER), d_dldi, d_dbg, sync);
 }
 
-// Host-to-device copy from a caller's buffer on the handle's stream,
-// staged when large.  The stage holds the data until the copy has run: a
-// later staged copy into the stage waits for it.
-void copy_in(pale_handle* h, void* dev, const void* host, size_t bytes) {
-  if (!bytes) return;
+struct DeviceIn {
+  void* dev;
+  const void* host;
+  size_t bytes;
+};
+
+// A staged copy's place in the stage.
+size_t stage_slot(size_t bytes) { return (bytes + 255) & ~size_t(255); }
+
+// Whether `total` bytes go through the stage.  With grow, the stage is made
+// as large; a query (rays, lookups) uses the stage that renders have left and
+// allocates none: pinning memory costs more than its copies save (14 MB, 10
+// ms), and a caller's first query counts.
+bool use_stage(pale_handle* h, size_t total, bool grow) {
+  if (total < kStageMinBytes) return false;
+  return grow ? h->stage.ensure(total, h->stream) : h->stage.p && h->stage.n >= total;
+}
+
+// Host-to-device copies from callers' buffers on the handle's stream,
+// staged when they add up to kStageMinBytes or more.  The stage holds the
+// data until the copies have run: a later staged copy into the stage waits
+// for them.
+void copy_in(pale_handle* h, const std::vector<DeviceIn>& ins, bool grow) {
   cudaStream_t s = h->stream;
-  if (bytes < kStageMinBytes) {
-    CK(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, s));
-    return;
-  }
-  if (h->stage.in_flight) {
+  size_t total = 0;
+  for (const DeviceIn& i : ins) total += stage_slot(i.bytes);
+  if (total >= kStageMinBytes && h->stage.in_flight) {
     CK(cudaStreamSynchronize(s));
     h->stage.in_flight = false;
   }
-  if (!h->stage.ensure(bytes, s)) {
-    CK(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, s));
-    return;
+  const bool staged = use_stage(h, total, grow);
+  std::vector<HostPiece> pieces;
+  size_t off = 0;
+  for (const DeviceIn& i : ins) {
+    if (staged && i.bytes) pieces.push_back(HostPiece{h->stage.p + off, static_cast<const char*>(i.host), i.bytes});
+    off += stage_slot(i.bytes);
   }
-  host_copy({HostPiece{h->stage.p, static_cast<const char*>(host), bytes}});
-  CK(cudaMemcpyAsync(dev, h->stage.p, bytes, cudaMemcpyHostToDevice, s));
-  h->stage.in_flight = true;
+  if (staged) host_copy(pieces);
+  off = 0;
+  for (const DeviceIn& i : ins) {
+    if (i.bytes) CK(cudaMemcpyAsync(i.dev, staged ? h->stage.p + off : i.host, i.bytes, cudaMemcpyHostToDevice, s));
+    off += stage_slot(i.bytes);
+  }
+  if (staged) h->stage.in_flight = true;
+}
+
+void copy_in(pale_handle* h, void* dev, const void* host, size_t bytes) {
+  copy_in(h, std::vector<DeviceIn>{DeviceIn{dev, host, bytes}}, true);
 }
 
 struct DeviceOut {
@@ -1436,13 +1464,12 @@ struct DeviceOut {
 // Device-to-host copies into callers' buffers: enqueued on the handle's
 // stream (through the stage when they add up to kStageMinBytes or more),
 // then the run state is read (with `stats`) and the stream synchronised.
-void copy_out(pale_handle* h, const std::vector<DeviceOut>& outs, bool stats) {
+void copy_out(pale_handle* h, const std::vector<DeviceOut>& outs, bool stats, bool grow = true) {
   cudaStream_t s = h->stream;
-  auto slot = [](size_t b) { return (b + 255) & ~size_t(255); };
   size_t total = 0;
   for (const DeviceOut& o : outs)
-    if (o.host && o.bytes) total += slot(o.bytes);
-  const bool staged = total >= kStageMinBytes && h->stage.ensure(total, s);
+    if (o.host && o.bytes) total += stage_slot(o.bytes);
+  const bool staged = use_stage(h, total, grow);
   std::vector<HostPiece> pieces;
   if (staged) {
     // (the copies into the stage run after any copy out of it: same stream)
@@ -1451,7 +1478,7 @@ void copy_out(pale_handle* h, const std::vector<DeviceOut>& outs, bool stats) {
       if (!o.host || !o.bytes) continue;
       CK(cudaMemcpyAsync(h->stage.p + off, o.dev, o.bytes, cudaMemcpyDeviceToHost, s));
       pieces.push_back(HostPiece{static_cast<char*>(o.host), h->stage.p + off, o.bytes});
-      off += slot(o.bytes);
+      off += stage_slot(o.bytes);
     }
   } else {
     for (const DeviceOut& o : outs)
@@ -2222,22 +2249,19 @@ int pale_trace_rays(pale_handle* h, uint32_t n, const float* o, const float* d, 
     if (!n) return PALE_OK;
     use_stream(h, h->own_stream);
     cudaStream_t s = h->stream;
-    DBuf<float> dO, dD, dT, dA, dP;
-    DBuf<int32_t> dI, dR;
-    dO.alloc(3ull * n); dD.alloc(3ull * n); dT.alloc(n); dA.alloc(n); dP.alloc(3ull * n); dI.alloc(n); dR.alloc(n);
-    CK(cudaMemcpyAsync(dO.p, o, 12ull * n, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(dD.p, d, 12ull * n, cudaMemcpyHostToDevice, s));
+    // inputs and outputs in the handle's query buffer: 6 and 7 words a ray
+    h->query.ensure(13ull * n);
+    float *dO = h->query.p, *dD = dO + 3ull * n, *dP = dD + 3ull * n, *dT = dP + 3ull * n, *dA = dT + n;
+    int32_t *dI = reinterpret_cast<int32_t*>(dA + n), *dR = dI + n;
+    copy_in(h, {DeviceIn{dO, o, 12ull * n}, DeviceIn{dD, d, 12ull * n}}, false);
     CK(cudaMemsetAsync(h->run.p, 0, sizeof(RunState), s));
-    trace_rays(h->view(), h->run.p, n, dO.p, dD.p, dI.p, dR.p, dT.p, dA.p, dP.p, s);
+    trace_rays(h->view(), h->run.p, n, dO, dD, dI, dR, dT, dA, dP, s);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(inst, dI.p, 4ull * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(prim, dR.p, 4ull * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(t, dT.p, 4ull * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(alpha, dA.p, 4ull * n, cudaMemcpyDeviceToHost, s));
-    if (pos) CK(cudaMemcpyAsync(pos, dP.p, 12ull * n, cudaMemcpyDeviceToHost, s));
     h->timed = 0;
     h->launches_last = 1;
-    copy_stats(h);
+    copy_out(h, {DeviceOut{inst, dI, 4ull * n}, DeviceOut{prim, dR, 4ull * n}, DeviceOut{t, dT, 4ull * n},
+                 DeviceOut{alpha, dA, 4ull * n}, DeviceOut{pos, dP, 12ull * n}},
+             true, false);
     return PALE_OK;
   });
 }
@@ -2250,20 +2274,17 @@ int pale_trace_transmittance(pale_handle* h, uint32_t n, const float* o, const f
     if (!n) return PALE_OK;
     use_stream(h, h->own_stream);
     cudaStream_t s = h->stream;
-    DBuf<float> dO, dD, dT, dX;
-    DBuf<int32_t> dI;
-    dO.alloc(3ull * n); dD.alloc(3ull * n); dT.alloc(n); dX.alloc(n); dI.alloc(n);
-    CK(cudaMemcpyAsync(dO.p, o, 12ull * n, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(dD.p, d, 12ull * n, cudaMemcpyHostToDevice, s));
+    h->query.ensure(9ull * n);
+    float *dO = h->query.p, *dD = dO + 3ull * n, *dT = dD + 3ull * n, *dX = dT + n;
+    int32_t* dI = reinterpret_cast<int32_t*>(dX + n);
+    copy_in(h, {DeviceIn{dO, o, 12ull * n}, DeviceIn{dD, d, 12ull * n}}, false);
     CK(cudaMemsetAsync(h->run.p, 0, sizeof(RunState), s));
-    trace_transmittance(h->view(), h->run.p, n, dO.p, dD.p, dI.p, dT.p, dX.p, s);
+    trace_transmittance(h->view(), h->run.p, n, dO, dD, dI, dT, dX, s);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(inst, dI.p, 4ull * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(t, dT.p, 4ull * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(transmit, dX.p, 4ull * n, cudaMemcpyDeviceToHost, s));
     h->timed = 0;
     h->launches_last = 1;
-    copy_stats(h);
+    copy_out(h, {DeviceOut{inst, dI, 4ull * n}, DeviceOut{t, dT, 4ull * n}, DeviceOut{transmit, dX, 4ull * n}}, true,
+             false);
     return PALE_OK;
   });
 }
@@ -2275,14 +2296,12 @@ int pale_gather_irradiance(pale_handle* h, uint32_t n, const float* pts, const f
     if (!n) return PALE_OK;
     use_stream(h, h->own_stream);
     cudaStream_t s = h->stream;
-    DBuf<float> dP, dN, dE;
-    dP.alloc(3ull * n); dN.alloc(3ull * n); dE.alloc(3ull * n);
-    CK(cudaMemcpyAsync(dP.p, pts, 12ull * n, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(dN.p, nrm, 12ull * n, cudaMemcpyHostToDevice, s));
-    gather_points(h->view(), n, dP.p, dN.p, dE.p, s);
+    h->query.ensure(9ull * n);
+    float *dP = h->query.p, *dN = dP + 3ull * n, *dE = dN + 3ull * n;
+    copy_in(h, {DeviceIn{dP, pts, 12ull * n}, DeviceIn{dN, nrm, 12ull * n}}, false);
+    gather_points(h->view(), n, dP, dN, dE, s);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(E, dE.p, 12ull * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    copy_out(h, {DeviceOut{E, dE, 12ull * n}}, false, false);
     return PALE_OK;
   });
 }

@@ -277,7 +277,7 @@ class Renderer:
         """Surfel parameters in BVH order (pale_bindings.cpp:733-850)."""
         out = N.PointsHolder(n=self.num_points)
         _check(self._lib, self._h, self._lib.pale_get_points(self._h, C.byref(out.struct)), "get_point_parameters")
-        return {k: out.arrays[k].copy() for k in POINT_FIELDS}
+        return {k: out.arrays[k] for k in POINT_FIELDS}   # this call's own arrays
 
     def get_point_order(self) -> np.ndarray:
         """order[bvh_index] = asset index of the last BVH build."""
@@ -332,7 +332,7 @@ class Renderer:
         if self._asset_stale:
             out = N.PointsHolder(n=self.num_points)
             _check(self._lib, self._h, self._lib.pale_get_asset(self._h, C.byref(out.struct)), "get_asset")
-            self._asset_host = {k: out.arrays[k].copy() for k in POINT_FIELDS}
+            self._asset_host = {k: out.arrays[k] for k in POINT_FIELDS}
             self._asset_stale = False
         return self._asset_host
 
@@ -561,8 +561,8 @@ class Renderer:
         o = np.ascontiguousarray(origins, np.float32).reshape(-1, 3)
         d = np.ascontiguousarray(directions, np.float32).reshape(-1, 3)
         n = o.shape[0]
-        inst, prim = np.zeros(n, np.int32), np.zeros(n, np.int32)
-        t, a, p = np.zeros(n, np.float32), np.zeros(n, np.float32), np.zeros((n, 3), np.float32)
+        inst, prim = np.empty(n, np.int32), np.empty(n, np.int32)
+        t, a, p = np.empty(n, np.float32), np.empty(n, np.float32), np.empty((n, 3), np.float32)
         rc = self._lib.pale_trace_rays(self._h, n, o.ctypes.data_as(N.f32p), d.ctypes.data_as(N.f32p),
                                        inst.ctypes.data_as(N.i32p), prim.ctypes.data_as(N.i32p),
                                        t.ctypes.data_as(N.f32p), a.ctypes.data_as(N.f32p), p.ctypes.data_as(N.f32p))
