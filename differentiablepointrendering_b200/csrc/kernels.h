@@ -373,6 +373,19 @@ constexpr int kLeafBatch = PALE_LEAF_BATCH;
 #endif
 constexpr int kKHitLeafBatch = PALE_KHIT_LEAF_BATCH;
 
+// Inner nodes a walk visits between two votes on leaf or node (measured at 1,
+// 2 and 3: closest hits 79.6, 79.2 and 80.1 ms on 200k surfels x 8 views,
+// 4.06, 3.90 and 3.79 ms on 50k; the 8-hit walk 58.0, 57.1 and 56.8 ms,
+// 1.64, 1.57 and 1.54 ms).
+#ifndef PALE_INNER_BURST
+#define PALE_INNER_BURST 2
+#endif
+constexpr int kInnerBurst = PALE_INNER_BURST;
+#ifndef PALE_KHIT_INNER_BURST
+#define PALE_KHIT_INNER_BURST 3
+#endif
+constexpr int kKHitInnerBurst = PALE_KHIT_INNER_BURST;
+
 #ifndef PALE_REFILL_STEPS
 #define PALE_REFILL_STEPS 16
 #endif

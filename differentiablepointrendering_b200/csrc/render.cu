@@ -396,6 +396,8 @@ __global__ void __launch_bounds__(kThreads, kWalkMinBlocks * (kBlock / kThreads)
   stage_top_nodes(A.scenes, s_top);
   const uint32_t n_in = A.st->active[parity];
   const int lane = threadIdx.x & 31;
+  const uint32_t lanes = walk_lanes(n_in, gridDim.x * (kThreads / 32));
+  const int batch = max(1, kLeafBatch * (int)lanes / 32);
   TravStack stk(s_top, A.scenes.n * A.scenes.staged);
   ClosestWalk w;
   TraceCounters ctr{0, 0};
@@ -403,14 +405,15 @@ __global__ void __launch_bounds__(kThreads, kWalkMinBlocks * (kBlock / kThreads)
   uint32_t cur = kInvalid;   // queue slot of this lane's ray
   bool more = true;          // uniform in the warp: the cursor has rays left
   for (;;) {
-    const unsigned need = __ballot_sync(0xffffffffu, cur == kInvalid);
+    const bool idle = cur == kInvalid && lane < lanes;
+    const unsigned need = __ballot_sync(0xffffffffu, idle);
     if (need && more) {
       const int leader = __ffs(need) - 1;
       uint32_t b0 = 0;
       if (lane == leader) b0 = atomicAdd(&A.st->walk_next, (uint32_t)__popc(need));
       b0 = __shfl_sync(0xffffffffu, b0, leader);
       if ((uint64_t)b0 + __popc(need) >= n_in) more = false;
-      if (cur == kInvalid) {
+      if (idle) {
         const uint32_t t = b0 + __popc(need & ((1u << lane) - 1u));
         if (t < n_in) {
           const float4 wa = A.tr.walkq[2 * (size_t)t], wb = A.tr.walkq[2 * (size_t)t + 1];
@@ -430,7 +433,7 @@ __global__ void __launch_bounds__(kThreads, kWalkMinBlocks * (kBlock / kThreads)
     for (int it = 0; it < kRefillSteps; ++it) {
       if (!__any_sync(0xffffffffu, cur != kInvalid)) break;
       const uint32_t sc = kMulti ? sid : 0u;
-      if (warp_step<kLeafBatch>(w, cur != kInvalid, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
+      if (warp_step<kInnerBurst>(w, cur != kInvalid, batch, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
           cur == kInvalid)
         continue;
       if (w.hit)
@@ -471,11 +474,11 @@ static void launch_walk(KernelT kernel, int threads, const Args& a, uint32_t arg
 }
 
 // The walk of the rays in queue `parity`: a persistent grid, every SM filled
-// once, no more blocks than `rays` rays need.
+// once, no more blocks than `rays` rays need at kMinWalkLanes a warp.
 static void ray_walk(const WalkArgs& w, uint32_t parity, uint32_t rays, cudaStream_t s) {
   const int wt = w.tr.walk_block == 64 || w.tr.walk_block == 128 ? (int)w.tr.walk_block : kBlock;
   const size_t smem = top_smem(w.scenes, wt);
-  const uint32_t nb = blocks_for(rays);
+  const uint32_t nb = blocks_for(rays, kBlock / 32 * kMinWalkLanes);
   if (w.scenes.n > 1) {
     if (wt == 64) launch_walk(k_ray_walk<true, 64>, 64, w, parity, smem, nb, s);
     else if (wt == 128) launch_walk(k_ray_walk<true, 128>, 128, w, parity, smem, nb, s);
@@ -898,6 +901,8 @@ __global__ void __launch_bounds__(kThreads, kRoundMinBlocks * (kBlock / kThreads
   stage_top_nodes(A.scenes, s_top);
   const uint32_t n = A.counts[round];
   const int lane = threadIdx.x & 31;
+  const uint32_t lanes = walk_lanes(n, gridDim.x * (kThreads / 32));
+  const int batch = max(1, kKHitLeafBatch * (int)lanes / 32);
   TravStack stk(s_top, A.scenes.n * A.scenes.staged);
 #if PALE_KHIT_SMEM
   KHitWalkS<K> w;
@@ -912,14 +917,15 @@ __global__ void __launch_bounds__(kThreads, kRoundMinBlocks * (kBlock / kThreads
   uint32_t cur = kInvalid;   // queue entry of this lane's walk
   bool more = true;          // uniform in the warp: the cursor has entries left
   for (;;) {
-    const unsigned need = __ballot_sync(0xffffffffu, cur == kInvalid);
+    const bool idle = cur == kInvalid && lane < lanes;
+    const unsigned need = __ballot_sync(0xffffffffu, idle);
     if (need && more) {
       const int leader = __ffs(need) - 1;
       uint32_t b0 = 0;
       if (lane == leader) b0 = atomicAdd(&A.st->walk_next, (uint32_t)__popc(need));
       b0 = __shfl_sync(0xffffffffu, b0, leader);
       if ((uint64_t)b0 + __popc(need) >= n) more = false;
-      if (cur == kInvalid) {
+      if (idle) {
         const uint32_t t = b0 + __popc(need & ((1u << lane) - 1u));
         if (t < n) {
           const float4 wa = A.walk[2 * (size_t)t], wb = A.walk[2 * (size_t)t + 1];
@@ -938,7 +944,7 @@ __global__ void __launch_bounds__(kThreads, kRoundMinBlocks * (kBlock / kThreads
     for (int it = 0; it < kRefillSteps; ++it) {
       if (!__any_sync(0xffffffffu, cur != kInvalid)) break;
       const uint32_t sc = kMulti ? sid : 0u;
-      if (warp_step<kKHitLeafBatch>(w, cur != kInvalid, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
+      if (warp_step<kKHitInnerBurst>(w, cur != kInvalid, batch, A.scenes.s[sc], s_top + sc * A.scenes.staged, stk, ctr, A.st) ||
           cur == kInvalid)
         continue;
       uint32_t rw[kKHitWords];

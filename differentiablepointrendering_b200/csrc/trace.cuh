@@ -449,20 +449,37 @@ struct KHitWalkS : WalkBase<KHitWalkS<K>> {
 };
 
 // One step of a persistent walk loop for the lanes of a warp: the lanes
-// whose walk stands at a leaf step together once at least kBatch of
-// them (or all of the walking lanes) do, the other times the lanes at inner
-// nodes step.  Returns for this lane whether its walk goes on (a lane that
-// sat out the step keeps walking).  Every lane of the warp calls it.
-template <int kBatch, class W>
-__device__ __forceinline__ bool warp_step(W& w, bool walking, const SceneView& S,
+// whose walk stands at a leaf step together once at least `batch` of them
+// (or all of the walking lanes) do, the other times the lanes at inner nodes
+// step, kBurst nodes at a time.  Returns for this lane whether its walk
+// goes on (a lane that sat out the step keeps walking).  Every lane of the
+// warp calls it.
+template <int kBurst, class W>
+__device__ __forceinline__ bool warp_step(W& w, bool walking, int batch, const SceneView& S,
                                           const TravNode* __restrict__ smem_top, TravStack& stk, TraceCounters& ctr,
                                           RunState* st) {
   const bool lf = walking && w.at_leaf();
   const unsigned ml = __ballot_sync(0xffffffffu, lf);
   const unsigned ma = __ballot_sync(0xffffffffu, walking);
-  const bool leaf_phase = ml != 0u && (ml == ma || __popc(ml) >= kBatch);
-  if (walking && lf == leaf_phase) return w.step(S, smem_top, stk, ctr, st);
+  const bool leaf_phase = ml != 0u && (ml == ma || __popc(ml) >= batch);
+  if (walking && lf == leaf_phase) {
+    bool on = w.step(S, smem_top, stk, ctr, st);
+#pragma unroll
+    for (int k = 1; k < kBurst; ++k)
+      if (!leaf_phase && on && !w.at_leaf()) on = w.step(S, smem_top, stk, ctr, st);
+    return on;
+  }
   return walking;
+}
+
+// The lanes of a warp that walk when `n` rays are shared by `warps` warps:
+// all of them, or, when the rays would not fill every warp, as many as give
+// each warp its share (a warp's lanes wait for one another at every step, so
+// few rays are walked faster spread over idle warps than packed into one).
+constexpr uint32_t kMinWalkLanes = 4;
+__device__ __forceinline__ uint32_t walk_lanes(uint32_t n, uint32_t warps) {
+  const uint32_t share = (n + warps - 1u) / warps;
+  return share >= 32u ? 32u : (share < kMinWalkLanes ? kMinWalkLanes : share);
 }
 
 // A 4x4 instance matrix (16 floats, 64 B aligned) in four 16-byte loads.
