@@ -497,7 +497,12 @@ __device__ __forceinline__ void load_matrix(const float* M, float (&m)[16]) {
 
 // The closest mesh hit, in object space per instance (intersectBLASMesh,
 // IntersectionKernels.h:37-105); `best` is the world distance of the hit
-// (+inf on a miss).
+// (+inf on a miss).  The boxes of up to 32 instances are tested first, then
+// each lane goes through the instances its own ray enters, in their order
+// and while their box is no farther than its closest hit: a ray enters one
+// or two of a room's walls, but the rays of a warp all of them, and testing
+// each instance as its box is met made the warp run every instance's
+// transform and triangles.
 __device__ __forceinline__ Hit intersect_meshes(const SceneView& S, V3 o, V3 d, V3 invw, float& best) {
   Hit h;
   h.inst = -1;
@@ -507,39 +512,49 @@ __device__ __forceinline__ Hit intersect_meshes(const SceneView& S, V3 o, V3 d, 
   h.pos = v3(0.f, 0.f, 0.f);
   best = __int_as_float(0x7f800000);
   const MeshView& M = S.mesh;
-  for (uint32_t i = 0; i < M.instances; ++i) {
+  auto enters = [&](uint32_t i) {
     const float4 lo = __ldg(&M.box[2 * i]), hi = __ldg(&M.box[2 * i + 1]);
-    if (!entered(slab_entry(o, invw, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, best), best)) continue;
-    float w2o[16];
-    load_matrix(M.w2o + 16 * i, w2o);
-    V3 oo = xform_point(w2o, o);
-    V3 dd = xform_dir(w2o, d);
-    uint2 rg = __ldg(&M.tri_range[i]);
-    float bt = __int_as_float(0x7f800000);
-    bool any = false;
-    uint32_t bprim = 0;
-    for (uint32_t k = 0; k < rg.y; ++k) {
-      const float4* tv = M.tri + 3 * (rg.x + k);
-      float t;
-      if (tri_hit(oo, dd, xyz(__ldg(&tv[0])), xyz(__ldg(&tv[1])), xyz(__ldg(&tv[2])), 1e-4f, t) && t < bt &&
-          t > 0.0f) {
-        bt = t;
-        any = true;
-        bprim = rg.x + k;
+    return entered(slab_entry(o, invw, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, best), best);
+  };
+  for (uint32_t base = 0; base < M.instances; base += 32) {
+    const uint32_t n = M.instances - base < 32u ? M.instances - base : 32u;
+    uint32_t mask = 0;
+    for (uint32_t k = 0; k < n; ++k) mask |= enters(base + k) ? 1u << k : 0u;
+    const float before = best;
+    for (; mask; mask &= mask - 1u) {
+      const uint32_t i = base + (__ffs(mask) - 1);
+      if (best < before && !enters(i)) continue;
+      float w2o[16];
+      load_matrix(M.w2o + 16 * i, w2o);
+      V3 oo = xform_point(w2o, o);
+      V3 dd = xform_dir(w2o, d);
+      uint2 rg = __ldg(&M.tri_range[i]);
+      float bt = __int_as_float(0x7f800000);
+      bool any = false;
+      uint32_t bprim = 0;
+      for (uint32_t k = 0; k < rg.y; ++k) {
+        const float4* tv = M.tri + 3 * (rg.x + k);
+        float t;
+        if (tri_hit(oo, dd, xyz(__ldg(&tv[0])), xyz(__ldg(&tv[1])), xyz(__ldg(&tv[2])), 1e-4f, t) && t < bt &&
+            t > 0.0f) {
+          bt = t;
+          any = true;
+          bprim = rg.x + k;
+        }
       }
-    }
-    if (!any) continue;
-    float o2w[16];
-    load_matrix(M.o2w + 16 * i, o2w);
-    V3 hw = xform_point(o2w, oo + scale(dd, bt));
-    float tw = dot(hw - o, d);
-    if (tw > 0.0f && tw < best) {
-      best = tw;
-      h.inst = (int)i;
-      h.t = tw;
-      h.pos = hw;
-      h.prim = bprim;
-      h.alpha = 0.0f;
+      if (!any) continue;
+      float o2w[16];
+      load_matrix(M.o2w + 16 * i, o2w);
+      V3 hw = xform_point(o2w, oo + scale(dd, bt));
+      float tw = dot(hw - o, d);
+      if (tw > 0.0f && tw < best) {
+        best = tw;
+        h.inst = (int)i;
+        h.t = tw;
+        h.pos = hw;
+        h.prim = bprim;
+        h.alpha = 0.0f;
+      }
     }
   }
   return h;
