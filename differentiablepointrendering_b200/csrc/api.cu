@@ -264,6 +264,7 @@ struct pale_handle {
   DBuf<uint4> vs_ent_b, sc_ent_b;
   DBuf<uint32_t> vs_base, vs_overflow, vs_chunk_base;
   DBuf<SceneGrads> vs_view_grads;   // per view gradient arrays of a per-view backward
+  DBuf<float> vs_terms;             // the sweep's terms, kSweepTerms per surfel of every scene entry
   uint64_t photon_gen = 0;     // photon maps traced or loaded so far
   uint64_t params_gen = 0;     // surfel parameter writes so far
   uint64_t bvh_gen = 0;        // BVH builds so far
@@ -1239,7 +1240,20 @@ void gather_adjoint(const std::vector<pale_handle*>& scenes, const std::vector<C
   for (size_t k = 0; k < scenes.size(); ++k) W.grads[k] = grads[k];
   W.all_grads = all ? 1 : 0;
   W.view_grads = d_view_grads;
+  if (all && !d_view_grads) {
+    size_t n = 0;
+    for (pale_handle* sk : scenes) n += sk->np;
+    h->vs_terms.ensure(kSweepTerms * n);
+    CK(cudaMemsetAsync(h->vs_terms.p, 0, kSweepTerms * n * sizeof(float), s));
+    n = 0;
+    for (size_t k = 0; k < scenes.size(); ++k) {
+      W.terms[k] = h->vs_terms.p + kSweepTerms * n;
+      n += scenes[k]->np;
+    }
+  }
   gather_backward(F, sel, h->vplan, W, scratch, s);
+  if (W.terms[0])
+    for (size_t k = 0; k < scenes.size(); ++k) unpack_gradients(W.terms[k], scenes[k]->np, grads[k], s);
   uint32_t stored = 0;
   uint64_t recs_all = 0, ents_all = 0;
   for (const VertexChunk& c : h->vplan.chunks) {

@@ -519,7 +519,13 @@ struct SweepArgs {
   // its scene's; a view whose opacity array is null is not swept
   const SceneGrads* view_grads;
   int all_grads;
+  // optional, with all_grads and without view_grads: per entry of `grads`
+  // kSweepTerms floats per surfel (zeroed by the caller) that the sweep adds
+  // into instead; k_grad_unpack then writes them to the gradient arrays
+  float* terms[kMaxScenes];
 };
+constexpr int kSweepTerms = 16;   // opacity, beta, position 3, tangent_u 3, tangent_v 3, scale 2, albedo 3
+void unpack_gradients(const float* terms, uint32_t n, const SceneGrads& out, cudaStream_t s);
 void gather_backward(const FrameArgs& a, const std::vector<CameraRec>& views, const VertexPlan& plan,
                      const SweepArgs& w, const VertexStore& scratch, cudaStream_t s);
 // Bins of a gather round of at most `entries` queue entries (two per

@@ -1891,18 +1891,21 @@ __device__ __forceinline__ float* sweep_target(const SceneGrads& G, uint32_t k, 
   }
 }
 
-constexpr int kSweepTerms = 16;   // opacity, beta, position 3, tangent_u 3, tangent_v 3, scale 2, albedo 3
-
 // One thread per entry; the layers of a warp's entries are visited by layer
 // index, deepest first, and the terms of lanes whose layer at that index
 // is the same surfel are added up inside the warp (__match_any_sync on the
-// scene and surfel, the lowest lane sums in lane order from shared memory)
-// before one atomicAdd per component, the components spread over lanes.
-// Neighbouring camera paths cross the same front surfels, so the first
-// layers of a warp share targets.
+// scene and surfel, in lane order from shared memory) before they go to
+// memory.  Neighbouring camera paths cross the same front surfels, so the
+// first layers of a warp share targets.  With every gradient group a surfel's
+// 16 terms lie side by side (SweepArgs::terms) and four lanes add them with a
+// 16-byte reduction each, eight surfels of a warp at a time: two sectors a
+// surfel and layer where the seven gradient arrays take seven, and no loop
+// over the surfels of a warp one by one.
 __global__ void __launch_bounds__(kBlock) k_vs_sweep(FrameArgs A, SweepArgs W, const uint32_t* __restrict__ base,
                                                      uint32_t round) {
-  __shared__ float s_val[kBlock / 32][kSweepTerms][33];
+  // per warp: a lane's terms in a row (20 floats apart: no bank conflicts)
+  __shared__ __align__(16) float s_val[kBlock / 32][32 * 20];
+  __shared__ uint32_t s_lead[kBlock / 32][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t e1 = base[kVertexBases + round + 1];
   const uint32_t e = base[kVertexBases + round] + blockIdx.x * kBlock + threadIdx.x;
@@ -1912,7 +1915,6 @@ __global__ void __launch_bounds__(kBlock) k_vs_sweep(FrameArgs A, SweepArgs W, c
     valid = false;
   }
   if (!__any_sync(0xffffffffu, valid)) return;
-  const int nterms = W.all_grads ? kSweepTerms : 1;
   float4 dT = make_float4(0.f, 0.f, 0.f, 1.f);
   uint4 b = make_uint4(0u, 0u, kInvalid, 0u);
   uint32_t sid = 0, route = 0, gp = 0;   // route: the gradient arrays' index (view or scene)
@@ -1966,7 +1968,7 @@ __global__ void __launch_bounds__(kBlock) k_vs_sweep(FrameArgs A, SweepArgs W, c
     }
   }
   const V3 dd = normalize(xyz(dT));
-  float (*val)[33] = s_val[wid];
+  float* val = s_val[wid];
 #pragma unroll
   for (int i = kGatherHits - 1; i >= 0; --i) {
     if (!__any_sync(0xffffffffu, i < ns)) continue;
@@ -1998,30 +2000,76 @@ __global__ void __launch_bounds__(kBlock) k_vs_sweep(FrameArgs A, SweepArgs W, c
       }
       Lb = scale(Lo, as[i]) + scale(Lb, 1.0f - as[i]);
     }
-    for (int c = 0; c < nterms; ++c) val[c][lane] = t[c];
+    if (W.all_grads) {
+      float4* row = reinterpret_cast<float4*>(val + 20 * lane);
+#pragma unroll
+      for (int c = 0; c < kSweepTerms / 4; ++c) row[c] = make_float4(t[4 * c], t[4 * c + 1], t[4 * c + 2], t[4 * c + 3]);
+    } else {
+      val[20 * lane] = t[0];
+    }
     __syncwarp();
     const unsigned grp = __match_any_sync(0xffffffffu, ((unsigned long long)route << 32) | k);
     const bool leader = k != kInvalid && lane == __ffs(grp) - 1;
-    if (leader && __popc(grp) > 1) {
-      for (int c = 0; c < nterms; ++c) {
+    const unsigned lm = __ballot_sync(0xffffffffu, leader);
+    if (!W.all_grads) {
+      if (leader) {
         float acc = 0.f;
-        for (unsigned r = grp; r; r &= r - 1u) acc += val[c][__ffs(r) - 1];
-        val[c][lane] = acc;
+        for (unsigned r = grp; r; r &= r - 1u) acc += val[20 * (__ffs(r) - 1)];
+        if (acc != 0.f) atomicAdd((W.view_grads ? W.view_grads[route] : W.grads[route]).opacity + k, acc);
       }
-    }
-    __syncwarp();
-    for (unsigned lm = __ballot_sync(0xffffffffu, leader); lm; lm &= lm - 1u) {
-      const int L = __ffs(lm) - 1;
-      const uint32_t kL = __shfl_sync(0xffffffffu, k, L);
-      const uint32_t rL = __shfl_sync(0xffffffffu, route, L);
-      if (lane < nterms) {
-        const float x = val[lane][L];
-        if (x != 0.f) atomicAdd(sweep_target(W.view_grads ? W.view_grads[rL] : W.grads[rL], kL, lane), x);
+    } else {
+      if (leader) s_lead[wid][__popc(lm & ((1u << lane) - 1u))] = lane;
+      __syncwarp();
+      const int leaders = __popc(lm);
+      for (int b0 = 0; b0 < leaders; b0 += 8) {
+        const int q = b0 + (lane >> 2);
+        const bool in = q < leaders;
+        const int L = in ? (int)s_lead[wid][q] : 0;
+        const uint32_t kL = __shfl_sync(0xffffffffu, k, L), rL = __shfl_sync(0xffffffffu, route, L);
+        const unsigned gL = __shfl_sync(0xffffffffu, grp, L);
+        if (!in) continue;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (unsigned r = gL; r; r &= r - 1u) {
+          const float4 y = reinterpret_cast<const float4*>(val + 20 * (__ffs(r) - 1))[lane & 3];
+          x = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+        }
+        if (W.terms[0]) {
+          if (x.x != 0.f || x.y != 0.f || x.z != 0.f || x.w != 0.f)
+            atomicAdd(reinterpret_cast<float4*>(W.terms[rL] + (size_t)kSweepTerms * kL) + (lane & 3), x);
+        } else {
+          const SceneGrads& G = W.view_grads ? W.view_grads[rL] : W.grads[rL];
+          const int c = 4 * (lane & 3);
+          if (x.x != 0.f) atomicAdd(sweep_target(G, kL, c), x.x);
+          if (x.y != 0.f) atomicAdd(sweep_target(G, kL, c + 1), x.y);
+          if (x.z != 0.f) atomicAdd(sweep_target(G, kL, c + 2), x.z);
+          if (x.w != 0.f) atomicAdd(sweep_target(G, kL, c + 3), x.w);
+        }
       }
     }
     __syncwarp();
   }
   if (valid) A.vs.ent_l[e] = make_float4(Lb.x, Lb.y, Lb.z, 0.f);
+}
+
+__global__ void __launch_bounds__(kBlock) k_grad_unpack(const float4* __restrict__ terms, uint32_t n, SceneGrads G) {
+  const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
+  if (k >= n) return;
+  float t[kSweepTerms];
+#pragma unroll
+  for (int c = 0; c < kSweepTerms / 4; ++c) {
+    const float4 x = terms[(size_t)(kSweepTerms / 4) * k + c];
+    t[4 * c] = x.x;
+    t[4 * c + 1] = x.y;
+    t[4 * c + 2] = x.z;
+    t[4 * c + 3] = x.w;
+  }
+#pragma unroll
+  for (int c = 0; c < kSweepTerms; ++c) *sweep_target(G, k, c) = t[c];
+}
+
+void unpack_gradients(const float* terms, uint32_t n, const SceneGrads& out, cudaStream_t s) {
+  if (n == 0) return;
+  k_grad_unpack<<<blocks_for(n), kBlock, 0, s>>>(reinterpret_cast<const float4*>(terms), n, out); note_launch();
 }
 
 void gather_backward(const FrameArgs& a0, const std::vector<CameraRec>& views, const VertexPlan& plan,
