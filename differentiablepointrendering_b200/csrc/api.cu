@@ -242,7 +242,7 @@ struct pale_handle {
   // K-hit walk result (kKHitWords words); then, in the same memory, the
   // round's lookups (per record 2 words, then 1)
   DBuf<float4> cg_entry;
-  DBuf<uint32_t> cg_bins;
+  DBuf<uint32_t> lookup_bins;      // of the camera's and the adjoint's lookups
   DBuf<uint32_t> cg_counts;
   DBuf<float4> cg_res, cg_fb;
   // run state, seeds, images, gradients
@@ -485,18 +485,21 @@ void size_wavefronts(pale_handle* h, uint64_t all_pix, uint32_t max_pix) {
     if (st.gradients == PALE_GRADIENTS_ALL) h->ev_ext.alloc(2 * qa);
     h->adj_hits.alloc(2 * qa);
     h->adj_walkq.alloc(2 * qa);
+    h->lookup_bins.ensure(gather_bins(h->adj_cap));
   }
   const uint64_t want = all_pix * std::max<uint32_t>(1u, st.gather_passes);
   const uint64_t cg_limit = st.gather_batch_paths ? st.gather_batch_paths : (1ull << 25);
-  const uint32_t path_cap =
-      (uint32_t)std::max<uint64_t>(std::max<uint64_t>(all_pix, 1), std::min<uint64_t>(want, cg_limit));
+  // (2^28 at most: a round's records stay below 2^31, the mark of the heavy
+  // lookups; a view is below 2^24 pixels, so a pass of it always fits)
+  const uint32_t path_cap = (uint32_t)std::min<uint64_t>(
+      std::max<uint64_t>(std::max<uint64_t>(all_pix, 1), std::min<uint64_t>(want, cg_limit)), 1ull << 28);
   if (path_cap > h->path_cap) {
     h->path_cap = path_cap;
     h->cg_paths.alloc(h->path_cap); h->cg_paths2.alloc(h->path_cap);
     h->cg_qrec.alloc(2 * (size_t)kGatherHits * h->path_cap); h->cg_res.alloc(h->path_cap);
     h->cg_info_a.alloc(h->path_cap); h->cg_info_b.alloc(h->path_cap);
     h->cg_entry.alloc(std::max<size_t>(3 + kKHitWords / 4, (3 * kGatherHits + 3) / 4) * (size_t)h->path_cap);
-    h->cg_bins.ensure(gather_bins(h->path_cap));
+    h->lookup_bins.ensure(gather_bins(h->path_cap));
   }
   h->cg_fb.ensure(std::max<uint64_t>(all_pix, 1));
 }
@@ -1017,10 +1020,8 @@ FrameArgs frame_args(const std::vector<pale_handle*>& scenes, uint32_t nsel, uin
   F.mhit = h->cg_entry.p;
   F.walk = F.mhit + h->path_cap;
   F.khit = reinterpret_cast<uint32_t*>(F.walk + 2 * (size_t)h->path_cap);
-  F.rec_bin = reinterpret_cast<uint2*>(h->cg_entry.p);
-  F.rec_order = reinterpret_cast<uint32_t*>(F.rec_bin + (size_t)kGatherHits * h->path_cap);
-  F.rec_heavy = reinterpret_cast<uint32_t*>(F.rec_bin);
-  F.bins = h->cg_bins.p;
+  uint2* bin = reinterpret_cast<uint2*>(h->cg_entry.p);
+  F.lookups = LookupOrder{bin, reinterpret_cast<uint32_t*>(bin + (size_t)kGatherHits * h->path_cap), h->lookup_bins.p, 0u};
   F.counts = h->cg_counts.p;
   F.res = h->cg_res.p;
   F.fb = h->cg_fb.p;
@@ -1362,6 +1363,8 @@ void adjoint_views(const std::vector<pale_handle*>& scenes, const std::vector<Vi
   A.light0_area = h->light0_area;
   A.timer = &h->timer;
   A.tr = TraceBufs{h->adj_hits.p, h->adj_walkq.p, st.walk_block};
+  uint2* bin = reinterpret_cast<uint2*>(h->adj_walkq.p);   // 8 + 4 of a slot's 32 bytes
+  A.lookups = LookupOrder{bin, reinterpret_cast<uint32_t*>(bin + h->adj_cap), h->lookup_bins.p, 0u};
   // jobs in the reference's order (view-major, then pass), packed into
   // batches of at most adj_cap paths and kMaxJobsPerBatch jobs
   const std::vector<uint32_t> slots = seed_slots(scenes, views);

@@ -234,9 +234,9 @@ struct RunState {
   uint32_t error;
   uint32_t walk_next;       // next ray of a persistent walk (sorted position)
   uint32_t lookup_next;     // lookups of the current round that find photons
-  uint32_t heavy_next;      // those of them that scan many photons
+  uint32_t heavy_count;     // those of them that scan many photons
+  uint32_t heavy_next;      // the next of these to be done
   uint32_t ray_next;        // rays placed in walk order (bin_offsets)
-  uint32_t pad;
   unsigned long long photon_segments;
   unsigned long long gather_segments;
   unsigned long long adjoint_segments;

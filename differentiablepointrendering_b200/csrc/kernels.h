@@ -250,6 +250,16 @@ struct VertexStore {
   int write;
 };
 
+// The photon lookups of a round or bounce, listed by grid cell: per item its
+// bin (a group of cells) and its rank in the bin, the items to look up in bin
+// order, and the bins: a power of two of counters, then offsets.
+struct LookupOrder {
+  uint2* bin;
+  uint32_t* order;
+  uint32_t* bins;
+  uint32_t mask;          // bins - 1 (set per call)
+};
+
 struct FrameArgs {
   SceneTable scenes;
   SceneSeeds sseeds[kMaxScenes];
@@ -290,15 +300,8 @@ struct FrameArgs {
   float4* walk;
   uint32_t* khit;
   // the round's lookups, written once the walk's buffers above have been
-  // read, in their memory: per record its bin (a group of grid cells) and
-  // its rank in the bin, and the records to look up, in bin order; bins is
-  // a power of two of counters, then offsets.  rec_heavy, the records left
-  // to the heavy lookups, takes the place of rec_bin.
-  uint2* rec_bin;
-  uint32_t* rec_order;
-  uint32_t* rec_heavy;
-  uint32_t* bins;
-  uint32_t bin_mask;       // bins - 1 (set per round)
+  // read, in their memory
+  LookupOrder lookups;
   KernelTimer* timer;      // host side, may be null
   // host side: a pinned word the length of the next round's queue is copied
   // to, and the event behind that copy
@@ -351,10 +354,6 @@ constexpr int kRoundMinBlocks = PALE_ROUND_MIN_BLOCKS;
 #define PALE_LOOKUP_MIN_BLOCKS 4
 #endif
 constexpr int kLookupMinBlocks = PALE_LOOKUP_MIN_BLOCKS;
-#ifndef PALE_HEAVY_MIN_BLOCKS
-#define PALE_HEAVY_MIN_BLOCKS 6
-#endif
-constexpr int kHeavyMinBlocks = PALE_HEAVY_MIN_BLOCKS;
 // The persistent walks (adjoint closest hit, camera 8 hits): lanes whose
 // walk has ended take a new ray every PALE_REFILL_STEPS node visits;
 // PALE_WALK_MIN_BLOCKS is the adjoint walk's register budget.
@@ -397,7 +396,7 @@ constexpr int kWalkMinBlocks = PALE_WALK_MIN_BLOCKS;
 // The adjoint transport kernel: its event record and gradient terms spill
 // at 64 registers.
 #ifndef PALE_TRANSPORT_MIN_BLOCKS
-#define PALE_TRANSPORT_MIN_BLOCKS 3
+#define PALE_TRANSPORT_MIN_BLOCKS 4
 #endif
 constexpr int kTransportMinBlocks = PALE_TRANSPORT_MIN_BLOCKS;
 
@@ -465,6 +464,8 @@ struct AdjointArgs {
   float light0_area;
   KernelTimer* timer;      // host side, may be null
   TraceBufs tr;
+  // the events' lookups, in the memory of the walk's records
+  LookupOrder lookups;
 };
 
 void photon_emit(const PhotonArgs& a, cudaStream_t s);

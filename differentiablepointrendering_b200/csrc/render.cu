@@ -862,7 +862,7 @@ __device__ __forceinline__ uint32_t vs_ent_slot(const FrameArgs& A, uint32_t rou
 // mesh distance plus intersect_scene's margin.
 __global__ void k_cg_mesh(FrameArgs A, uint32_t round) {
   const uint32_t n = A.counts[round];
-  if (blockIdx.x == 0 && threadIdx.x == 0) A.st->walk_next = A.st->lookup_next = A.st->heavy_next = 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) A.st->walk_next = A.st->lookup_next = A.st->heavy_count = A.st->heavy_next = 0u;
   const RayRec* __restrict__ in = A.paths[round & 1];
   for (uint32_t slot = blockIdx.x * kBlock + threadIdx.x; slot < n; slot += gridDim.x * kBlock) {
     const float4 ro = in[slot].o;
@@ -1129,31 +1129,45 @@ __global__ void __launch_bounds__(kBlock, kTraceMinBlocks) k_cg_round(FrameArgs 
   warp_count(&A.st->gather_segments, segs);
 }
 
-// Round step 2: the photon lookups of the round's records.  Most layers see
-// no photon at all (on a lit box of 200k surfels 68% of the camera lookups,
-// the cloud being dark away from the light) and most photons are scanned by
-// the few lookups near the light (95% of them by lookups of more than 256
-// photons), so the records are split three ways:
-// - k_cg_lit (a thread per record) finishes those whose window holds no
+// Kinds of adjoint interactions and events.
+enum : uint32_t { kKindNone = 0, kKindNull = 1, kKindReflect = 2, kKindTransmit = 3, kKindProjection = 4 };
+
+// Whether an event (its kind, target, material, pixel) needs the irradiance
+// at its point.  A null event ending on a surfel has no material (the
+// reference reads materials[0xFFFFFFFF], AdjointKernels.cpp:446-447): no
+// contribution.
+__device__ __forceinline__ bool event_looks_up(const uint4& d) {
+  return d.x == kKindProjection || d.x == kKindReflect || (d.x == kKindNull && d.z != kInvalid);
+}
+
+// Photon lookups, of a gather round's records (round step 2) and of an
+// adjoint bounce's events.  Most see no photon at all (on a lit box of 200k
+// surfels 68% of the camera lookups, the cloud being dark away from the
+// light) and most photons are scanned by the few near the light (95% of them
+// by lookups of more than 256 photons), so they are split three ways:
+// - k_lookup_lit (a thread per lookup) finishes those whose window holds no
 //   photon, from one bit per grid cell, and lists the others, in the order
 //   of their grid cells when there are enough of them to share photons: a
-//   counting sort into bins (the cell modulo the number of bins; a record's
+//   counting sort into bins (the cell modulo the number of bins; a lookup's
 //   rank in its bin is the counter it found), k_bin_offsets making offsets
-//   of the counts and k_cg_order placing the records;
-// - k_cg_lookup does the short ones, kLookupLanes lanes each, and lists
-//   those of more than kLookupHeavy photons;
-// - k_cg_lookup_heavy does these, a warp each.
+//   of the counts and k_lookup_order placing the lookups;
+// - k_lookup does the short ones, kLookupLanes lanes each, and marks those
+//   of more than kLookupHeavy photons;
+// - k_lookup_heavy does these, a warp each, from the list k_lookup_list makes.
 // The order inside a bin and between blocks of bins depends on timing, the
 // results do not: each lookup reads its own window alone.  On 200k surfels x
-// 8 views the lookups of a step took 173 ms with a warp per record, 78 ms
-// so: 37 ms the heavy ones, which wait on L1 and L2 (11 TB/s of photon
-// records read by the SMs), 36 ms the short ones (63% of the issue slots),
-// 5 ms the split.
-// Queue entries of a round from which its lookups are grouped by grid cell:
-// the grouping costs three short launches (9 us when nothing is there to
-// group) and, on 200k surfels x 8 views, 4.9 ms against the 6.7 ms that the
-// shared photons save (lookups 36.9 -> 30.2 ms, the heavy ones alike).
+// 8 views the camera lookups of a step took 173 ms with a warp per record.
+
+// From how many queue entries a round's lookups (or paths a bounce's events)
+// are grouped by grid cell: the grouping costs three short launches (9 us
+// when nothing is there to group) and, on 200k surfels x 8 views, 4.9 ms
+// against the 6.7 ms that the shared photons save (short lookups 36.9 -> 30.2
+// ms, the heavy ones alike).
 constexpr uint32_t kSortEntries = 32768;
+
+// Marks a lookup of the order as left to the heavy lookups (lookups are
+// below 2^28).
+constexpr uint32_t kHeavyMark = 0x80000000u;
 
 // The radiance a layer adds to its path: Lo * weight.
 __device__ __forceinline__ float4 layer_radiance(const SceneView& S, uint32_t kind, uint32_t idx, V3 E, float weight) {
@@ -1168,127 +1182,258 @@ __device__ __forceinline__ float4 layer_radiance(const SceneView& S, uint32_t ki
   return make_float4(c.x, c.y, c.z, 0.f);
 }
 
-template <bool kMulti, bool kSort>
-__global__ void __launch_bounds__(kBlock) k_cg_lit(FrameArgs A, uint32_t round) {
-  const uint32_t n = A.counts[kMaxLayers + 2 + round];
+// The lookups of a gather round: a record's point, normal and index word; a
+// lookup's result is the layer's contribution, over the record's first float4.
+struct RoundLookups {
+  FrameArgs A;
+  uint32_t round;
+  struct Keep {
+    float weight, word;
+  };
+  __device__ __forceinline__ const SceneTable& scenes() const { return A.scenes; }
+  __device__ __forceinline__ RunState* state() const { return A.st; }
+  __device__ __forceinline__ uint32_t count() const { return A.counts[kMaxLayers + 2 + round]; }
+  // lookup i; false for an unused record
+  template <bool kMulti>
+  __device__ __forceinline__ bool get(uint32_t i, V3& x, V3& n, uint32_t& sid, Keep& keep) const {
+    const float4 rb = A.qrec[2 * (size_t)i + 1];
+    const uint32_t word = __float_as_uint(rb.w);
+    if ((word >> 30) == kRecNone) return false;
+    const float4 ra = A.qrec[2 * (size_t)i];
+    x = xyz(ra);
+    n = xyz(rb);
+    sid = kMulti ? (word >> 27) & 7u : 0u;
+    keep = Keep{ra.w, rb.w};
+    return true;
+  }
+  __device__ __forceinline__ void put(uint32_t i, V3 E, uint32_t sid, const Keep& keep) const {
+    const uint32_t word = __float_as_uint(keep.word);
+    A.qrec[2 * (size_t)i] = layer_radiance(A.scenes.s[sid], word >> 30, word & kRecIndexMask, E, keep.weight);
+    const uint32_t vr = vs_rec_slot(A, round, i);
+    if (vr != kInvalid) A.vs.rec_ew[vr] = make_float4(E.x, E.y, E.z, keep.word);
+  }
+  __device__ __forceinline__ void tally(uint32_t queries, uint32_t scanned) const {
+    warp_count(&A.st->gather_queries, queries);
+    warp_count(&A.st->photons_scanned, scanned);
+    warp_count(&A.st->gather_photons_scanned, scanned);
+  }
+};
+
+// The lookups of a bounce's events (k_transport's): the event's point and
+// normal; a lookup's irradiance takes the normal's place.
+struct EventLookups {
+  AdjointArgs A;
+  using Keep = float;
+  __device__ __forceinline__ const SceneTable& scenes() const { return A.scenes; }
+  __device__ __forceinline__ RunState* state() const { return A.st; }
+  __device__ __forceinline__ uint32_t count() const { return A.st->event_count; }
+  // event i; false when it has no lookup
+  template <bool kMulti>
+  __device__ __forceinline__ bool get(uint32_t i, V3& x, V3& n, uint32_t& sid, Keep& keep) const {
+    const EventRec* ev = A.ev.list + i;
+    if (!event_looks_up(ev->d)) return false;
+    const float4 b = ev->b;
+    x = xyz(ev->a);
+    n = xyz(b);
+    sid = kMulti ? A.cams[A.jobs[__float_as_uint(ev->c.w)].cam].scene : 0u;
+    keep = b.w;
+    return true;
+  }
+  __device__ __forceinline__ void put(uint32_t i, V3 E, uint32_t, const Keep& keep) const {
+    A.ev.list[i].b = make_float4(E.x, E.y, E.z, keep);
+  }
+  __device__ __forceinline__ void tally(uint32_t queries, uint32_t scanned) const {
+    warp_count(&A.st->gather_queries, queries);
+    warp_count(&A.st->photons_scanned, scanned);
+  }
+};
+
+template <class Lookups, bool kMulti, bool kSort>
+__global__ void __launch_bounds__(kBlock) k_lookup_lit(Lookups Q, LookupOrder so) {
+  const uint32_t n = Q.count();
   const int lane = threadIdx.x & 31;
   uint32_t queries = 0;
   for (uint32_t b = blockIdx.x * kBlock; b < n; b += gridDim.x * kBlock) {
     const uint32_t i = b + threadIdx.x;
-    uint32_t bin = kInvalid;
-    if (i < n) {
-      const float4 rb = A.qrec[2 * (size_t)i + 1];
-      const uint32_t word = __float_as_uint(rb.w), kind = word >> 30;
-      if (kind != kRecNone) {
-        const float4 ra = A.qrec[2 * (size_t)i];
-        const uint32_t sid = kMulti ? (word >> 27) & 7u : 0u;
-        const SceneView& S = A.scenes.s[sid];
-        ++queries;
-        if (window_lit(S.grid, xyz(ra))) {
-          bin = 0;
-          if (kSort) {
-            int c[3];
-            world_to_cell(S.grid, xyz(ra), c);
-            bin = ((uint32_t)((c[2] * S.grid.res[1] + c[1]) * S.grid.res[0] + c[0]) + sid * 0x9E3779B1u) & A.bin_mask;
-          }
-        } else {
-          const V3 E = v3(0.f, 0.f, 0.f);
-          A.qrec[2 * (size_t)i] = layer_radiance(S, kind, word & kRecIndexMask, E, ra.w);
-          const uint32_t vr = vs_rec_slot(A, round, i);
-          if (vr != kInvalid) A.vs.rec_ew[vr] = make_float4(0.f, 0.f, 0.f, rb.w);
+    uint32_t bin = kInvalid, sid = 0;
+    V3 x, nrm;
+    typename Lookups::Keep keep;
+    if (i < n && Q.template get<kMulti>(i, x, nrm, sid, keep)) {
+      const GridView& G = Q.scenes().s[sid].grid;
+      ++queries;
+      if (window_lit(G, x)) {
+        bin = 0;
+        if (kSort) {
+          int c[3];
+          world_to_cell(G, x, c);
+          bin = ((uint32_t)((c[2] * G.res[1] + c[1]) * G.res[0] + c[0]) + sid * 0x9E3779B1u) & so.mask;
         }
+      } else {
+        Q.put(i, v3(0.f, 0.f, 0.f), sid, keep);
       }
     }
     if (kSort) {
-      const uint32_t rank = bin_rank(A.bins, bin);
-      if (i < n) A.rec_bin[i] = make_uint2(bin, rank);
+      const uint32_t rank = bin_rank(so.bins, bin);
+      if (i < n) so.bin[i] = make_uint2(bin, rank);
     } else {
       const unsigned lit = __ballot_sync(0xffffffffu, bin != kInvalid);
       uint32_t base = 0;
-      if (lit && lane == 0) base = atomicAdd(&A.st->lookup_next, (uint32_t)__popc(lit));
+      if (lit && lane == 0) base = atomicAdd(&Q.state()->lookup_next, (uint32_t)__popc(lit));
       base = __shfl_sync(0xffffffffu, base, 0);
-      if (bin != kInvalid) A.rec_order[base + __popc(lit & ((1u << lane) - 1u))] = i;
+      if (bin != kInvalid) so.order[base + __popc(lit & ((1u << lane) - 1u))] = i;
     }
   }
-  warp_count(&A.st->gather_queries, queries);
+  Q.tally(queries, 0u);
 }
 
-__global__ void __launch_bounds__(kBlock) k_cg_order(FrameArgs A, uint32_t round) {
-  const uint32_t n = A.counts[kMaxLayers + 2 + round];
+template <class Lookups>
+__global__ void __launch_bounds__(kBlock) k_lookup_order(Lookups Q, LookupOrder so) {
+  const uint32_t n = Q.count();
   for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
-    const uint2 b = A.rec_bin[i];
-    if (b.x != kInvalid) A.rec_order[A.bins[b.x] + b.y] = i;
+    const uint2 b = so.bin[i];
+    if (b.x != kInvalid) so.order[so.bins[b.x] + b.y] = i;
   }
 }
 
-// A group's first lane writes the layer's contribution over the record's
-// first float4.
-template <bool kMulti>
-__global__ void __launch_bounds__(kBlock, kLookupMinBlocks) k_cg_lookup(FrameArgs A, uint32_t round) {
-  __shared__ uint32_t s_list[kBlock / kLookupLanes][kLookupList];
-  __shared__ float s_sq[kBlock / kLookupLanes][16];
+// A group's first lane writes the result.
+template <class Lookups, bool kMulti>
+__global__ void __launch_bounds__(kBlock, kLookupMinBlocks) k_lookup(Lookups Q, LookupOrder so) {
+  __shared__ LaneLookup s_lane[kBlock / kLookupLanes];
   __shared__ GatherConst s_gc[kMaxScenes];
-  if (threadIdx.x < A.scenes.n) s_gc[threadIdx.x] = gather_const(A.scenes.s[threadIdx.x].grid);
+  if (threadIdx.x < Q.scenes().n) s_gc[threadIdx.x] = gather_const(Q.scenes().s[threadIdx.x].grid);
   __syncthreads();
-  const uint32_t n = A.st->lookup_next;
+  const uint32_t n = Q.state()->lookup_next;
   const uint32_t g = threadIdx.x / kLookupLanes, groups = gridDim.x * (kBlock / kLookupLanes);
   uint32_t scanned = 0;
   for (uint32_t b = blockIdx.x * (kBlock / kLookupLanes) + g; __any_sync(0xffffffffu, b < n); b += groups) {
     const bool valid = b < n;
-    uint32_t i = 0;
-    float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rb = ra;
+    uint32_t i = 0, sid = 0;
+    V3 x = v3(0.f, 0.f, 0.f), nrm = x;
+    typename Lookups::Keep keep{};
     if (valid) {
-      i = A.rec_order[b];
-      ra = A.qrec[2 * (size_t)i];
-      rb = A.qrec[2 * (size_t)i + 1];
+      i = so.order[b];
+      Q.template get<kMulti>(i, x, nrm, sid, keep);
     }
-    const uint32_t word = __float_as_uint(rb.w);
-    const uint32_t sid = kMulti ? (word >> 27) & 7u : 0u;
-    const SceneView& S = A.scenes.s[sid];
     uint32_t cnt = 0;
     bool heavy;
-    const V3 E = gather_irradiance_lanes<kLookupLanes>(S.grid, s_gc[sid], xyz(ra), xyz(rb), valid, s_list[g],
-                                                       s_sq[g], cnt, heavy);
+    const uint32_t sc = kMulti ? sid : 0u;
+    const V3 E = gather_irradiance_lanes<kLookupLanes>(Q.scenes().s[sc].grid, s_gc[sc], x, nrm, valid, s_lane[g], cnt,
+                                                       heavy);
     if (valid && threadIdx.x % kLookupLanes == 0) {
       if (heavy) {
-        A.rec_heavy[atomicAdd(&A.st->heavy_next, 1u)] = i;
+        so.order[b] = i | kHeavyMark;
       } else {
         scanned += cnt;
-        A.qrec[2 * (size_t)i] = layer_radiance(S, word >> 30, word & kRecIndexMask, E, ra.w);
-        const uint32_t vr = vs_rec_slot(A, round, i);
-        if (vr != kInvalid) A.vs.rec_ew[vr] = make_float4(E.x, E.y, E.z, rb.w);
+        Q.put(i, E, sc, keep);
       }
     }
   }
-  warp_count(&A.st->photons_scanned, scanned);
-  warp_count(&A.st->gather_photons_scanned, scanned);
+  Q.tally(0u, scanned);
 }
 
-template <bool kMulti>
-__global__ void __launch_bounds__(kBlock, kHeavyMinBlocks) k_cg_lookup_heavy(FrameArgs A, uint32_t round) {
+// The heavy lookups of the order, listed in its order (up to the order of
+// the blocks) in the memory of the bins' ranks, which are no longer needed.
+__global__ void __launch_bounds__(kBlock) k_lookup_list(RunState* st, LookupOrder so) {
+  __shared__ uint32_t s_warp[kBlock / 32], s_base;
+  const uint32_t n = st->lookup_next;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t* list = reinterpret_cast<uint32_t*>(so.bin);
+  for (uint32_t b = blockIdx.x * kBlock; b < n; b += gridDim.x * kBlock) {
+    const uint32_t r = b + threadIdx.x < n ? so.order[b + threadIdx.x] : 0u;
+    const bool heavy = (r & kHeavyMark) != 0u;
+    const unsigned m = __ballot_sync(0xffffffffu, heavy);
+    if (!__syncthreads_or(m != 0u)) continue;
+    if (lane == 0) s_warp[wid] = __popc(m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t t = 0;
+      for (int w = 0; w < kBlock / 32; ++w) {
+        const uint32_t c = s_warp[w];
+        s_warp[w] = t;
+        t += c;
+      }
+      s_base = atomicAdd(&st->heavy_count, t);
+    }
+    __syncthreads();
+    if (heavy) list[s_base + s_warp[wid] + __popc(m & ((1u << lane) - 1u))] = r & ~kHeavyMark;
+    __syncthreads();
+  }
+}
+
+// Two blocks of 16 warps per SM, whose warps take neighbouring lookups (a
+// range of the list at a time, handed out one by one), so that they read the
+// same photons and many loads hit L1.  What bounds them is the SM's load
+// path: 36 bytes a photon, eleven or twelve 128-byte wavefronts a round of 32
+// photons, 14e9 photons a step of 200k surfels x 8 views in 34.9 ms, 74% of
+// one wavefront a cycle.  (36.9 ms with six blocks of 8 warps anywhere on
+// the list; one block of 32 warps 35.5 ms, rounds aligned to 32 photons, four
+// wavefronts a load but up to twice the rounds of a short row, 43 ms.)
+constexpr int kHeavyThreads = 512;
+constexpr int kHeavyBlocks = 2;
+constexpr uint32_t kHeavyRange = 128;
+
+template <class Lookups, bool kMulti>
+__global__ void __launch_bounds__(kHeavyThreads, kHeavyBlocks) k_lookup_heavy(Lookups Q, LookupOrder so) {
   __shared__ GatherConst s_gc[kMaxScenes];
-  if (threadIdx.x < A.scenes.n) s_gc[threadIdx.x] = gather_const(A.scenes.s[threadIdx.x].grid);
-  __syncthreads();
-  const uint32_t n = A.st->heavy_next;
+  __shared__ uint32_t s_first, s_next;
+  if (threadIdx.x < Q.scenes().n) s_gc[threadIdx.x] = gather_const(Q.scenes().s[threadIdx.x].grid);
+  const uint32_t n = Q.state()->heavy_count;
+  const uint32_t* list = reinterpret_cast<const uint32_t*>(so.bin);
   const int lane = threadIdx.x & 31;
+  // smaller ranges, down to a lookup per warp, when there is little to share
+  uint32_t range = kHeavyRange;
+  while (range > kHeavyThreads / 32u && (uint64_t)range * gridDim.x * 4u > n) range >>= 1;
   uint32_t scanned = 0;
-  for (uint32_t b = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); b < n; b += gridDim.x * (kBlock / 32)) {
-    const uint32_t i = A.rec_heavy[b];
-    const float4 ra = A.qrec[2 * (size_t)i], rb = A.qrec[2 * (size_t)i + 1];
-    const uint32_t word = __float_as_uint(rb.w);
-    const uint32_t sid = kMulti ? (word >> 27) & 7u : 0u;
-    const SceneView& S = A.scenes.s[sid];
-    uint32_t cnt = 0;
-    const V3 E = gather_irradiance_rows(S.grid, s_gc[sid], xyz(ra), xyz(rb), cnt);
-    if (lane == 0) {
-      scanned += cnt;
-      A.qrec[2 * (size_t)i] = layer_radiance(S, word >> 30, word & kRecIndexMask, E, ra.w);
-      const uint32_t vr = vs_rec_slot(A, round, i);
-      if (vr != kInvalid) A.vs.rec_ew[vr] = make_float4(E.x, E.y, E.z, rb.w);
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_first = s_next = atomicAdd(&Q.state()->heavy_next, range);
+    __syncthreads();
+    const uint32_t first = s_first;
+    if (first >= n) break;
+    const uint32_t end = n - first < range ? n : first + range;
+    for (;;) {
+      uint32_t k = 0;
+      if (lane == 0) k = atomicAdd(&s_next, 1u);
+      k = __shfl_sync(0xffffffffu, k, 0);
+      if (k >= end) break;
+      const uint32_t i = list[k];
+      uint32_t sid = 0, cnt = 0;
+      V3 x, nrm;
+      typename Lookups::Keep keep;
+      if (!Q.template get<kMulti>(i, x, nrm, sid, keep)) continue;
+      const uint32_t sc = kMulti ? sid : 0u;
+      const V3 E = gather_irradiance_rows(Q.scenes().s[sc].grid, s_gc[sc], x, nrm, cnt);
+      if (lane == 0) {
+        scanned += cnt;
+        Q.put(i, E, sc, keep);
+      }
     }
   }
-  warp_count(&A.st->photons_scanned, scanned);
-  warp_count(&A.st->gather_photons_scanned, scanned);
+  Q.tally(0u, scanned);
+}
+
+// The lookups of Q: `items` bounds the items of the call (records, events),
+// `entries` what their grouping is judged and sized by.
+template <class Lookups, bool kMulti>
+static void run_lookups(const Lookups& Q, RunState* st, LookupOrder so, uint64_t items, uint32_t entries,
+                        cudaStream_t s) {
+  int dev = 0, sms = 148, per_sm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lookup<Lookups, kMulti>, kBlock, 0);
+  const uint32_t grid = std::min<uint32_t>((uint32_t)sms * 8u, blocks_for(items));
+  if (entries >= kSortEntries) {
+    so.mask = gather_bins(entries) - 1u;
+    cudaMemsetAsync(so.bins, 0, ((size_t)so.mask + 1) * sizeof(uint32_t), s);
+    k_lookup_lit<Lookups, kMulti, true><<<grid, kBlock, 0, s>>>(Q, so); note_launch();
+    k_bin_offsets<<<(so.mask + 1u) / (kBlock * kBinItems), kBlock, 0, s>>>(so.bins, &st->lookup_next); note_launch();
+    k_lookup_order<<<grid, kBlock, 0, s>>>(Q, so); note_launch();
+  } else {
+    k_lookup_lit<Lookups, kMulti, false><<<grid, kBlock, 0, s>>>(Q, so); note_launch();
+  }
+  k_lookup<Lookups, kMulti><<<(uint32_t)std::max(1, sms * std::max(1, per_sm)), kBlock, 0, s>>>(Q, so); note_launch();
+  k_lookup_list<<<grid, kBlock, 0, s>>>(st, so); note_launch();
+  k_lookup_heavy<Lookups, kMulti><<<(uint32_t)std::max(1, sms * kHeavyBlocks), kHeavyThreads, 0, s>>>(Q, so); note_launch();
 }
 
 // Round step 3: one lane per entry adds its layers' contributions in order
@@ -1470,7 +1615,7 @@ namespace {
 
 // The launch shapes of the camera gather's kernels.
 struct GatherShape {
-  uint32_t grid_r = 1, grid_l = 1, grid_h = 1, grid_b = 1;
+  uint32_t grid_r = 1;
   int wt = kBlock;
   size_t smem = 0;
 };
@@ -1479,25 +1624,20 @@ template <bool kMulti>
 GatherShape gather_shape(const FrameArgs& a) {
   GatherShape g;
   // persistent grids: every SM filled once
-  int dev = 0, sms = 148, per_sm_l = 1, per_sm_h = 1, per_sm_r = 1;
+  int dev = 0, sms = 148, per_sm_r = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   g.wt = a.walk_block == 64 || a.walk_block == 128 ? (int)a.walk_block : kBlock;
   g.smem = top_smem(a.scenes, g.wt) + (PALE_KHIT_SMEM ? (size_t)kGatherHits * g.wt * sizeof(uint2) : 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_r, k_cg_round<kGatherHits>, kBlock, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_l, k_cg_lookup<kMulti>, kBlock, 0);
   g.grid_r = (uint32_t)std::max(1, sms * std::max(1, per_sm_r));
-  g.grid_l = (uint32_t)std::max(1, sms * std::max(1, per_sm_l));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_h, k_cg_lookup_heavy<kMulti>, kBlock, 0);
-  g.grid_h = (uint32_t)std::max(1, sms * std::max(1, per_sm_h));
-  g.grid_b = (uint32_t)std::max(1, sms * 8);
   return g;
 }
 
 // The rounds of one chunk of n paths (its view_start already on the
 // device); returns the rounds run.
 template <bool kMulti>
-uint32_t gather_rounds(FrameArgs a, const GatherShape& g, uint32_t n, cudaStream_t s) {
+uint32_t gather_rounds(const FrameArgs& a, const GatherShape& g, uint32_t n, cudaStream_t s) {
   cudaMemsetAsync(a.counts, 0, 2 * (kMaxLayers + 2) * sizeof(uint32_t), s);
   k_cg_init<<<blocks_for(n), kBlock, 0, s>>>(a, n); note_launch();
   // every round consumes at least one layer of each live path, so
@@ -1518,17 +1658,7 @@ uint32_t gather_rounds(FrameArgs a, const GatherShape& g, uint32_t n, cudaStream
     cudaMemcpyAsync(const_cast<uint32_t*>(a.h_live), a.counts + round + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
     cudaEventRecord(a.round_ev, s);
     if (a.timer) a.timer->begin(kTimeLookup, s);
-    if (live >= kSortEntries) {
-      a.bin_mask = gather_bins(live) - 1u;
-      cudaMemsetAsync(a.bins, 0, ((size_t)a.bin_mask + 1) * sizeof(uint32_t), s);
-      k_cg_lit<kMulti, true><<<g.grid_b, kBlock, 0, s>>>(a, round); note_launch();
-      k_bin_offsets<<<(a.bin_mask + 1u) / (kBlock * kBinItems), kBlock, 0, s>>>(a.bins, &a.st->lookup_next); note_launch();
-      k_cg_order<<<g.grid_b, kBlock, 0, s>>>(a, round); note_launch();
-    } else {
-      k_cg_lit<kMulti, false><<<std::min(g.grid_b, blocks_for((uint64_t)live * kGatherHits)), kBlock, 0, s>>>(a, round); note_launch();
-    }
-    k_cg_lookup<kMulti><<<g.grid_l, kBlock, 0, s>>>(a, round); note_launch();
-    k_cg_lookup_heavy<kMulti><<<g.grid_h, kBlock, 0, s>>>(a, round); note_launch();
+    run_lookups<RoundLookups, kMulti>(RoundLookups{a, round}, a.st, a.lookups, (uint64_t)live * kGatherHits, live, s);
     if (a.timer) a.timer->end(s);
     k_cg_compose<<<blocks_for(live), kBlock, 0, s>>>(a, round); note_launch();
     ++round;
@@ -1598,7 +1728,6 @@ void camera_gather(const FrameArgs& a, const std::vector<CameraRec>& views, uint
 }
 
 // ------------------------------------------------------------- adjoint
-enum : uint32_t { kKindNone = 0, kKindNull = 1, kKindReflect = 2, kKindTransmit = 3, kKindProjection = 4 };
 
 // launchRayGenAdjointKernel (AdjointKernels.cpp:15-84) + the per-spp
 // reset of the pending states (SyclBridge.cpp:222), for every job of a batch.
@@ -1645,7 +1774,7 @@ __global__ void k_adj_raygen(AdjointArgs A, uint32_t npaths) {
 // with it): k_adj_mesh, k_ray_walk, and k_adj_bounce reading their records.
 __global__ void k_adj_mesh(AdjointArgs A, uint32_t parity) {
   const uint32_t slot = blockIdx.x * kBlock + threadIdx.x;
-  if (slot == 0) A.st->walk_next = A.st->event_count = 0u;
+  if (slot == 0) A.st->walk_next = A.st->event_count = A.st->lookup_next = A.st->heavy_count = A.st->heavy_next = 0u;
   if (slot >= A.st->active[parity]) return;
   const float4 rd = A.qb.q[parity][slot].d;
   const uint32_t sid = A.cams[A.jobs[__float_as_uint(rd.w) >> 8].cam].scene;
@@ -2117,6 +2246,10 @@ void gather_backward(const FrameArgs& a0, const std::vector<CameraRec>& views, c
 // per component, the components of one group spread over lanes.
 constexpr int kTransportTerms = 16;   // opacity, beta, position 3, tangent_u 3, tangent_v 3, scale 2, albedo 3 - 1
 
+// kLookups: with the lookups (each by the whole warp, one after another);
+// else they were run before (EventLookups) and an event holds its irradiance
+// in the place of its normal.
+template <bool kLookups>
 __global__ void __launch_bounds__(kBlock, kTransportMinBlocks) k_transport(AdjointArgs A) {
   __shared__ float4 s_terms[kBlock];                        // per warp: the lookups' row compaction
   __shared__ float s_val[kBlock / 32][kTransportTerms + 1][33];   // per warp: the lanes' terms
@@ -2154,14 +2287,11 @@ __global__ void __launch_bounds__(kBlock, kTransportMinBlocks) k_transport(Adjoi
       ev.d = make_uint4(kInvalid, kInvalid, kInvalid, 0u);
     }
     const uint32_t kind = ev.d.x;
-    // a null event ending on a surfel has no material (the reference reads
-    // materials[0xFFFFFFFF], AdjointKernels.cpp:446-447): no contribution
-    const bool need =
-        valid && (kind == kKindProjection || kind == kKindReflect || (kind == kKindNull && ev.d.z != kInvalid));
-    if (need) ++queries;
-    V3 E = v3(0.f, 0.f, 0.f);
-    const bool lit = need && window_lit(A.scenes.s[sid].grid, xyz(ev.a));
-    for (unsigned m = __ballot_sync(0xffffffffu, lit); m; m &= m - 1u) {
+    const bool need = valid && event_looks_up(ev.d);
+    V3 E = need && !kLookups ? xyz(ev.b) : v3(0.f, 0.f, 0.f);
+    if (kLookups && need) ++queries;
+    const bool lit = kLookups && need && window_lit(A.scenes.s[sid].grid, xyz(ev.a));
+    for (unsigned m = kLookups ? __ballot_sync(0xffffffffu, lit) : 0u; m; m &= m - 1u) {
       const int j = __ffs(m) - 1;
       const V3 xj = v3(__shfl_sync(0xffffffffu, ev.a.x, j), __shfl_sync(0xffffffffu, ev.a.y, j),
                        __shfl_sync(0xffffffffu, ev.a.z, j));
@@ -2298,6 +2428,13 @@ void adjoint_raygen(const AdjointArgs& a, uint32_t npaths, cudaStream_t s) {
   k_adj_raygen<<<blocks_for(std::max<uint32_t>(npaths, kMaxJobsPerBatch)), kBlock, 0, s>>>(a, npaths); note_launch();
 }
 
+// Paths of a batch from which its events' lookups are taken out of the
+// transport, into the kernels of the camera's lookups: their launches cost
+// about 20 us a bounce, the lookups inside the transport 27 ms of a step of
+// 200k surfels x 8 views against 17 ms outside, 5.2 against 3.1 ms of 393k
+// paths over dense photons, 0.32 against 0.32 ms of 262k paths over sparse
+// ones.
+constexpr uint32_t kSplitPaths = 131072u;
 // One bounce of every job of the batch; npaths bounds the live queue.
 void adjoint_bounce(AdjointArgs a, uint32_t bounce, bool last, uint32_t npaths, cudaStream_t s) {
   const uint32_t nb = blocks_for(npaths);
@@ -2323,9 +2460,16 @@ void adjoint_bounce(AdjointArgs a, uint32_t bounce, bool last, uint32_t npaths, 
                                   JobScan{a.job_count + next, a.job_start + next, a.njobs}); note_launch();
   k_queue_scatter<<<nb, kBlock, 0, s>>>(a, parity, 0, 0u); note_launch();
   // a warp per tile of 32 events: a grid that fills every SM once
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_transport, kBlock, 0);
   if (a.timer) a.timer->begin(kTimeTransport, s);
-  k_transport<<<(uint32_t)std::max(1, sms * std::max(1, per_sm)), kBlock, 0, s>>>(a); note_launch();
+  if (npaths >= kSplitPaths) {
+    if (a.scenes.n > 1) run_lookups<EventLookups, true>(EventLookups{a}, a.st, a.lookups, npaths, npaths, s);
+    else run_lookups<EventLookups, false>(EventLookups{a}, a.st, a.lookups, npaths, npaths, s);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_transport<false>, kBlock, 0);
+    k_transport<false><<<(uint32_t)std::max(1, sms * std::max(1, per_sm)), kBlock, 0, s>>>(a); note_launch();
+  } else {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_transport<true>, kBlock, 0);
+    k_transport<true><<<(uint32_t)std::max(1, sms * std::max(1, per_sm)), kBlock, 0, s>>>(a); note_launch();
+  }
   if (a.timer) a.timer->end(s);
 }
 

@@ -834,6 +834,9 @@ __device__ __forceinline__ void clip_row(const GridView& G, const GatherConst& G
   }
 }
 
+// Rounds of a row in flight (2 and 4 measured 36.4 and 35.5 ms, 7.9 and 7.1 ms
+// over dense photons).
+constexpr int kHeavyUnroll = 4;
 // gatherDiffuseIrradianceAtPoint (KernelHelpers.h:990-1037), done by a
 // whole warp for one query (x, n), which every lane passes.  Photons are
 // stored sorted by cell with ascending deposit index inside a cell, and the
@@ -879,7 +882,7 @@ __device__ __forceinline__ V3 gather_irradiance_rows(const GridView& G, const Ga
       const int k = __ffs(nm) - 1;
       const uint32_t rj0 = __shfl_sync(0xffffffffu, j0, k), rend = __shfl_sync(0xffffffffu, end, k);
       const uint32_t rturn = __shfl_sync(0xffffffffu, turn, k);
-#pragma unroll 2
+#pragma unroll kHeavyUnroll
       for (uint32_t j = rj0 + ((lane + rturn - rj0) & 31u); j < rend; j += 32) {
         const float4 pa = __ldg(&G.pa[j]), pb = __ldg(&G.pb[j]);
         const float pc = __ldg(&G.pc[j]);
@@ -1031,15 +1034,14 @@ __device__ __forceinline__ bool window_lit(const GridView& G, V3 x) {
 // lane, the others by shuffles), so the result is that function's, bit for
 // bit.  What it saves is the per-query work, most of a short lookup's
 // instructions: window corners, row clipping, scan and butterfly run for
-// 32 / kLanes queries at once, and a lane reads its photon numbers from a
-// list its group expands from the rows (`list`, kLookupList words per
-// group), so that short rows leave no lane idle: on lookups of up to 256
-// photons about 240 warp instructions a lookup against 380 by a whole warp.
-// The photon numbers of neighbouring queries are neighbours when the queries
-// are grouped by cell (L1 hits 52 -> 77%).  A query of more
-// than kLookupHeavy photons is not done (heavy; its result is undefined):
-// there the photons' own work counts, which a whole warp shares better.
-constexpr int kLookupList = 64;
+// 32 / kLanes queries at once, and a lane finds a photon's row by counting,
+// in a word of bits, the rows that start up to it (the rows' first photons
+// stand in shared memory), so that short rows leave no lane idle: on lookups
+// of up to 256 photons about 190 warp instructions a lookup against 380 by a
+// whole warp.  The photon numbers of neighbouring queries are neighbours when
+// the queries are grouped by cell (L1 hits 52 -> 77%).  A query of more than
+// kLookupHeavy photons is not done (heavy; its result is undefined): there
+// the photons' own work counts, which a whole warp shares better.
 // (128, 256 and 512 measured 77, 73 and 73 ms of lookups on 200k surfels, 8
 // views; 1.61, 1.50 and 1.56 ms on six small ones)
 #ifndef PALE_LOOKUP_HEAVY
@@ -1047,10 +1049,18 @@ constexpr int kLookupList = 64;
 #endif
 constexpr uint32_t kLookupHeavy = PALE_LOOKUP_HEAVY;
 
+// Shared memory of a group's lookup: per non-empty row its first photon less
+// its place in the sequence; a bit per photon of the sequence, set where a
+// row starts; squared distances to the window's y rows and z slabs.
+struct LaneLookup {
+  uint32_t row[32];
+  uint32_t starts[kLookupHeavy / 32];
+  float sq[16];
+};
+
 template <int kLanes>
 __device__ __forceinline__ V3 gather_irradiance_lanes(const GridView& G, const GatherConst& GC, V3 x, V3 n,
-                                                      bool valid, uint32_t* list, float* sq, uint32_t& count,
-                                                      bool& heavy) {
+                                                      bool valid, LaneLookup& sm, uint32_t& count, bool& heavy) {
   constexpr int kSlots = 32 / kLanes;   // partial sums per lane, and rows per lane of 32
   const int p = threadIdx.x & (kLanes - 1);
   const float r = G.radius, r2 = r * r;
@@ -1092,7 +1102,7 @@ __device__ __forceinline__ V3 gather_irradiance_lanes(const GridView& G, const G
     float dd = 0.f;
     if (c > 0) dd = fmaxf(dd, (o + (float)c * ce - 0.01f * ce) - xa);
     if (c < ra - 1) dd = fmaxf(dd, xa - (o + (float)(c + 1) * ce + 0.01f * ce));
-    sq[i] = dd * dd;
+    sm.sq[i] = dd * dd;
   }
   __syncwarp();
   float ax[kSlots], ay[kSlots], az[kSlots];
@@ -1111,7 +1121,7 @@ __device__ __forceinline__ V3 gather_irradiance_lanes(const GridView& G, const G
       if (k < rows) {
         const int kz = (int)(((float)k + 0.5f) * inv_ny);
         const int ky = k - kz * ny;
-        const float rho2 = sq[ky & 7] + sq[8 + (kz & 7)];
+        const float rho2 = sm.sq[ky & 7] + sm.sq[8 + (kz & 7)];
         if (rho2 <= reach2) {
           const float q = fmaxf(reach2 - rho2, 1e-30f);
           const float w = q * rsqrtf(q) * 1.001f + 0.01f * G.cell.x;
@@ -1131,74 +1141,84 @@ __device__ __forceinline__ V3 gather_irradiance_lanes(const GridView& G, const G
         }
       }
     }
+    // places in the sequence (lengths in the low half, non-empty rows in the
+    // high half; a lane's length stops at 4095, which is heavy already)
+    uint32_t ne = 0;
 #pragma unroll
-    for (int t = 0; t < kSlots; ++t) tot += len[t];
-    uint32_t ex = tot;
+    for (int t = 0; t < kSlots; ++t) {
+      tot += len[t] < 4095u ? len[t] : 4095u;
+      ne += len[t] != 0u ? 1u : 0u;
+    }
+    const uint32_t own = (tot < 4095u ? tot : 4095u) | (ne << 16);
+    uint32_t ex = own;
 #pragma unroll
     for (int o = 1; o < kLanes; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, ex, o, kLanes);
       if (p >= o) ex += y;
     }
-    uint32_t seq = __shfl_sync(0xffffffffu, ex, kLanes - 1, kLanes);
-    ex -= tot;
+    uint32_t seq = __shfl_sync(0xffffffffu, ex, kLanes - 1, kLanes) & 0xFFFFu;
+    ex -= own;
     if (seq > kLookupHeavy) heavy = true;
-    if (heavy) {
-      seq = 0;
-#pragma unroll
-      for (int t = 0; t < kSlots; ++t) len[t] = 0;
-    }
+    if (heavy) seq = 0;
     scanned += seq;
     const uint32_t most = __reduce_max_sync(0xffffffffu, seq);
-    for (uint32_t wb = 0; wb < most; wb += kLookupList) {
-      // the window's photon numbers
-      const uint32_t we = wb + kLookupList;
+    if (most == 0u) continue;
+#pragma unroll
+    for (uint32_t w = 0; w < kLookupHeavy / 32; w += kLanes)
+      if (w + p < kLookupHeavy / 32) sm.starts[w + p] = 0u;
+    __syncwarp();
+    {
+      uint32_t v = ex & 0xFFFFu, k = ex >> 16;
 #pragma unroll
       for (int t = 0; t < kSlots; ++t) {
-        while (len[t] != 0u && ex < we) {
-          list[ex - wb] = j0[t];
-          ++ex;
-          ++j0[t];
-          --len[t];
+        if (len[t] != 0u && v < seq) {
+          sm.row[k] = j0[t] - v;
+          atomicOr(&sm.starts[v >> 5], 1u << (v & 31u));
+          ++k;
+          v += len[t];
         }
       }
-      __syncwarp();
-      const uint32_t stop = most < we ? most : we;
-      for (uint32_t b = wb; b < stop; b += 32) {
-        constexpr int kAhead = kSlots < 4 ? kSlots : 4;   // photons loaded at once
-#pragma unroll
-        for (int s0 = 0; s0 < kSlots; s0 += kAhead) {
-          if (b + s0 * kLanes >= stop) break;
-          float4 pa[kAhead];
-          uint32_t j[kAhead];
-#pragma unroll
-          for (int s = 0; s < kAhead; ++s) {
-            const uint32_t v = b + (s0 + s) * kLanes + p;
-            pa[s] = make_float4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);   // fails the radius test
-            j[s] = 0;
-            if (v < seq) {
-              j[s] = list[v - wb];
-              pa[s] = __ldg(&G.pa[j[s]]);
-            }
-          }
-#pragma unroll
-          for (int s = 0; s < kAhead; ++s) {
-            const float dx = pa[s].x - x.x, dy = pa[s].y - x.y, dz = pa[s].z - x.z;
-            const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
-            if (d2 <= r2) {
-              const float4 pb = __ldg(&G.pb[j[s]]);
-              const float pc = __ldg(&G.pc[j[s]]);
-              const float cosine = -__fmaf_rn(n.z, pb.z, __fmaf_rn(n.y, pb.y, n.x * pb.x));
-              if (!(cosine < 0.0f)) {
-                ax[s0 + s] = __fmaf_rn(pa[s].w, invArea, ax[s0 + s]);
-                ay[s0 + s] = __fmaf_rn(pb.w, invArea, ay[s0 + s]);
-                az[s0 + s] = __fmaf_rn(pc, invArea, az[s0 + s]);
-              }
-            }
-          }
-        }
-      }
-      __syncwarp();
     }
+    __syncwarp();
+    uint32_t before = 0xFFFFFFFFu;   // rows that start before the block, less one
+    for (uint32_t b = 0; b < most; b += 32) {
+      const uint32_t starts = sm.starts[b >> 5];
+      constexpr int kAhead = kSlots < 4 ? kSlots : 4;   // photons loaded at once
+#pragma unroll
+      for (int s0 = 0; s0 < kSlots; s0 += kAhead) {
+        if (b + s0 * kLanes >= most) break;
+        float4 pa[kAhead];
+        uint32_t j[kAhead];
+#pragma unroll
+        for (int s = 0; s < kAhead; ++s) {
+          const int l = (s0 + s) * kLanes + p;
+          const uint32_t v = b + l;
+          pa[s] = make_float4(__int_as_float(0x7f800000), 0.f, 0.f, 0.f);   // fails the radius test
+          j[s] = 0;
+          if (v < seq) {
+            j[s] = v + sm.row[before + __popc(starts & (0xFFFFFFFFu >> (31 - l)))];
+            pa[s] = __ldg(&G.pa[j[s]]);
+          }
+        }
+#pragma unroll
+        for (int s = 0; s < kAhead; ++s) {
+          const float dx = pa[s].x - x.x, dy = pa[s].y - x.y, dz = pa[s].z - x.z;
+          const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
+          if (d2 <= r2) {
+            const float4 pb = __ldg(&G.pb[j[s]]);
+            const float pc = __ldg(&G.pc[j[s]]);
+            const float cosine = -__fmaf_rn(n.z, pb.z, __fmaf_rn(n.y, pb.y, n.x * pb.x));
+            if (!(cosine < 0.0f)) {
+              ax[s0 + s] = __fmaf_rn(pa[s].w, invArea, ax[s0 + s]);
+              ay[s0 + s] = __fmaf_rn(pb.w, invArea, ay[s0 + s]);
+              az[s0 + s] = __fmaf_rn(pc, invArea, az[s0 + s]);
+            }
+          }
+        }
+      }
+      before += __popc(starts);
+    }
+    __syncwarp();
   }
   count += scanned;
 #pragma unroll

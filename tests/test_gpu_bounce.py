@@ -34,7 +34,8 @@ def test_photon_pass_matches_oracle(gpu, photons, surfels):
 
 
 @pytest.mark.parametrize("gradients", ["opacity", "all"])
-@pytest.mark.parametrize("res", [16, 90, 129])     # 512, 16200 and 33282 adjoint paths
+# 512, 16200, 33282 and 135200 adjoint paths (the last: lookups apart from the transport)
+@pytest.mark.parametrize("res", [16, 90, 129, 260])
 def test_adjoint_matches_oracle(gpu, res, gradients):
     scene = make_box_scene(900, cameras=1, resolution=res)
     st = {"photons": 20000, "bounces": 3, "forward_passes": 1, "gather_passes": 1, "adjoint_bounces": 4,
