@@ -355,8 +355,13 @@ constexpr int kRoundMinBlocks = PALE_ROUND_MIN_BLOCKS;
 #endif
 constexpr int kLookupMinBlocks = PALE_LOOKUP_MIN_BLOCKS;
 // The persistent walks (adjoint closest hit, camera 8 hits): lanes whose
-// walk has ended take a new ray every PALE_REFILL_STEPS node visits;
-// PALE_WALK_MIN_BLOCKS is the adjoint walk's register budget.
+// walk has ended take a new ray every PALE_REFILL_STEPS node visits.
+// PALE_WALK_MIN_BLOCKS and PALE_WALK_MANY_BLOCKS are the closest-hit walk's
+// register budgets for few and for many rays: with many, its warps wait for
+// the next node's load a quarter of the time, and a fifth block (48
+// registers, 8 B spilled) hides more of that than the spill costs.  At 4, 5
+// and 6 blocks, with 8 stack entries in shared memory, 79.1, 74.8 and 82.9 ms
+// on 200k surfels x 8 views (60 B spilled at 6).
 // A persistent walk's lanes standing at leaves test them together once at
 // least PALE_LEAF_BATCH lanes of the warp do (or every walking lane);
 // PALE_KHIT_LEAF_BATCH for the camera's 8-hit walk, whose rays meet more
@@ -393,6 +398,10 @@ constexpr int kRefillSteps = PALE_REFILL_STEPS;
 #define PALE_WALK_MIN_BLOCKS 4
 #endif
 constexpr int kWalkMinBlocks = PALE_WALK_MIN_BLOCKS;
+#ifndef PALE_WALK_MANY_BLOCKS
+#define PALE_WALK_MANY_BLOCKS 5
+#endif
+constexpr int kWalkManyBlocks = PALE_WALK_MANY_BLOCKS;
 // The adjoint transport kernel: its event record and gradient terms spill
 // at 64 registers.
 #ifndef PALE_TRANSPORT_MIN_BLOCKS

@@ -389,8 +389,8 @@ struct WalkArgs {
 // while walks of very different lengths end.  A walk that finds a surfel
 // ends with one store of it and its distance in the ray's hit record; the
 // hits do not depend on the schedule.
-template <bool kMulti, int kThreads>
-__global__ void __launch_bounds__(kThreads, kWalkMinBlocks * (kBlock / kThreads))
+template <bool kMulti, int kThreads, int kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks * (kBlock / kThreads))
     k_ray_walk(WalkArgs A, uint32_t parity) {
   extern __shared__ TravNode s_top[];
   stage_top_nodes(A.scenes, s_top);
@@ -475,19 +475,28 @@ static void launch_walk(KernelT kernel, int threads, const Args& a, uint32_t arg
 
 // The walk of the rays in queue `parity`: a persistent grid, every SM filled
 // once, no more blocks than `rays` rays need at kMinWalkLanes a warp.
+template <bool kMulti, int kBlocks>
 static void ray_walk(const WalkArgs& w, uint32_t parity, uint32_t rays, cudaStream_t s) {
   const int wt = w.tr.walk_block == 64 || w.tr.walk_block == 128 ? (int)w.tr.walk_block : kBlock;
   const size_t smem = top_smem(w.scenes, wt);
   const uint32_t nb = blocks_for(rays, kBlock / 32 * kMinWalkLanes);
-  if (w.scenes.n > 1) {
-    if (wt == 64) launch_walk(k_ray_walk<true, 64>, 64, w, parity, smem, nb, s);
-    else if (wt == 128) launch_walk(k_ray_walk<true, 128>, 128, w, parity, smem, nb, s);
-    else launch_walk(k_ray_walk<true, 256>, 256, w, parity, smem, nb, s);
-  } else {
-    if (wt == 64) launch_walk(k_ray_walk<false, 64>, 64, w, parity, smem, nb, s);
-    else if (wt == 128) launch_walk(k_ray_walk<false, 128>, 128, w, parity, smem, nb, s);
-    else launch_walk(k_ray_walk<false, 256>, 256, w, parity, smem, nb, s);
-  }
+  if (wt == 64) launch_walk(k_ray_walk<kMulti, 64, kBlocks>, 64, w, parity, smem, nb, s);
+  else if (wt == 128) launch_walk(k_ray_walk<kMulti, 128, kBlocks>, 128, w, parity, smem, nb, s);
+  else launch_walk(k_ray_walk<kMulti, 256, kBlocks>, 256, w, parity, smem, nb, s);
+}
+
+// The fifth block pays for one scene's many rays.  With 4 and 5 blocks:
+// 16M rays of 200k surfels (12 bounces) 76.3 and 72.8 ms, 1M of 200k 3.52
+// and 3.45 ms (6 bounces), 1M of 20k 18.1 and 17.9 ms (36 bounces); but 100k
+// and 262k rays of 10k surfels (8 bounces) 1.26 and 1.40 ms, where a warp has
+// few rays and the walks' own length counts, and three scenes' rays 17.2 and
+// 18.3 ms, whose staged nodes leave the fifth block little L1.
+constexpr uint32_t kManyRays = 1u << 19;
+
+static void ray_walk(const WalkArgs& w, uint32_t parity, uint32_t rays, cudaStream_t s) {
+  if (w.scenes.n > 1) ray_walk<true, kWalkMinBlocks>(w, parity, rays, s);
+  else if (rays < kManyRays) ray_walk<false, kWalkMinBlocks>(w, parity, rays, s);
+  else ray_walk<false, kWalkManyBlocks>(w, parity, rays, s);
 }
 
 // --------------------------------------------------------------- photons
