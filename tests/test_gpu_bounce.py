@@ -33,6 +33,12 @@ def test_photon_pass_matches_oracle(gpu, photons, surfels):
     assert first == 0 or close.mean() > 0.99
 
 
+@pytest.mark.parametrize("photons", [(1 << 19) - 1, 1 << 19, (1 << 19) + 33])
+def test_walk_of_many_rays_matches_oracle(gpu, photons):
+    # on both sides of the queue size from which the walk has its own build
+    test_photon_pass_matches_oracle(gpu, photons, 700)
+
+
 @pytest.mark.parametrize("gradients", ["opacity", "all"])
 # 512, 16200, 33282 and 135200 adjoint paths (the last: lookups apart from the transport)
 @pytest.mark.parametrize("res", [16, 90, 129, 260])
