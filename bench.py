@@ -126,8 +126,8 @@ class ClockSampler:
 # 36 B per photon scanned and 8 B (two cell offsets) per grid row of its
 # window (25 rows); the adjoint bounce also reads and writes its 48 B
 # pending state, and its three kernels (mesh pass, persistent walk,
-# shading) pass 128 B of hit and walk records per ray between them (written
-# 64 B, read 48 + 16 B); a gradient event is a 64 B record, its lookup and
+# shading) pass 128 B of hit and walk records per ray between them (two 32 B
+# records, each written and read); a gradient event is a 64 B record, its lookup and
 # an 8 B atomic read-modify-write.
 ROWS_PER_QUERY = 25
 FWD_COUNTERS = ("photon_segments", "photons_stored", "gather_segments", "gather_node_visits", "gather_surfel_tests",
