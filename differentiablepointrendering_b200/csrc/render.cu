@@ -771,7 +771,7 @@ __device__ __forceinline__ void primary_ray(const CameraRec& C, float px, float 
 // trace's own hit; a surfel that is not hit from the chained origin, e.g.
 // within 1e-4 behind the previous layer, is passed over as the layered walk
 // passes over it); a round that used all K continues from the last one.
-// Every layer's photon lookup becomes a record; k_cg_lookup gives each
+// Every layer's photon lookup becomes a record; the lookup kernels give each
 // record a warp, and k_cg_compose adds a path's contributions in layer order,
 // so the sums are the layered walk's.  The walk draws no random numbers, so
 // queue order does not matter.  Each finished path writes its radiance to
@@ -829,7 +829,7 @@ __global__ void k_cg_init(FrameArgs A, uint32_t n) {
 
 // Lookup record (2 x float4): (position, weight) (lookup normal, index |
 // kind << 30), weight = T * alpha for a surfel layer, T for the diffuse mesh
-// that ends a path.  k_cg_lookup overwrites the first float4 with the
+// that ends a path.  The lookup overwrites the first float4 with the
 // layer's radiance contribution.  Unused slots of an entry's range are
 // kRecNone with zero contribution.
 // The index word also holds the record's scene: index (27 bits) | scene
