@@ -771,8 +771,8 @@ __device__ __forceinline__ void primary_ray(const CameraRec& C, float px, float 
 // trace's own hit; a surfel that is not hit from the chained origin, e.g.
 // within 1e-4 behind the previous layer, is passed over as the layered walk
 // passes over it); a round that used all K continues from the last one.
-// Every layer's photon lookup becomes a record; the lookup kernels give each
-// record a warp, and k_cg_compose adds a path's contributions in layer order,
+// Every layer's photon lookup becomes a record, which the lookup kernels
+// answer, and k_cg_compose adds a path's contributions in layer order,
 // so the sums are the layered walk's.  The walk draws no random numbers, so
 // queue order does not matter.  Each finished path writes its radiance to
 // res[path]; k_cg_finalize then adds the passes of a pixel in pass order,
