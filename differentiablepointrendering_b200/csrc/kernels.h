@@ -531,7 +531,7 @@ struct SweepArgs {
   int all_grads;
   // optional, with all_grads and without view_grads: per entry of `grads`
   // kSweepTerms floats per surfel (zeroed by the caller) that the sweep adds
-  // into instead; k_grad_unpack then writes them to the gradient arrays
+  // into instead; k_grad_unpack then adds them to the gradient arrays
   float* terms[kMaxScenes];
 };
 constexpr int kSweepTerms = 16;   // opacity, beta, position 3, tangent_u 3, tangent_v 3, scale 2, albedo 3

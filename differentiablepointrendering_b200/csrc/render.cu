@@ -2189,6 +2189,8 @@ __global__ void __launch_bounds__(kBlock) k_vs_sweep(FrameArgs A, SweepArgs W, c
   if (valid) A.vs.ent_l[e] = make_float4(Lb.x, Lb.y, Lb.z, 0.f);
 }
 
+// Adds the sweep's terms to the gradient arrays: entries of a call may name
+// the same arrays, which then hold the sum.
 __global__ void __launch_bounds__(kBlock) k_grad_unpack(const float4* __restrict__ terms, uint32_t n, SceneGrads G) {
   const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
   if (k >= n) return;
@@ -2202,7 +2204,8 @@ __global__ void __launch_bounds__(kBlock) k_grad_unpack(const float4* __restrict
     t[4 * c + 3] = x.w;
   }
 #pragma unroll
-  for (int c = 0; c < kSweepTerms; ++c) *sweep_target(G, k, c) = t[c];
+  for (int c = 0; c < kSweepTerms; ++c)
+    if (t[c] != 0.f) *sweep_target(G, k, c) += t[c];
 }
 
 void unpack_gradients(const float* terms, uint32_t n, const SceneGrads& out, cudaStream_t s) {

@@ -138,3 +138,33 @@ def test_five_scenes_in_one_wavefront_equal_each_alone(gpu):
     finally:
         for r in rs:
             r.close()
+
+
+@pytest.mark.parametrize("estimator", ["reference", "gather"])
+def test_entries_that_share_gradient_arrays_hold_the_sum(gpu, estimator):
+    """The same surfels under two lights (two scenes), one view each: with the
+    same output arrays these hold what the entries' own arrays add up to,
+    every group."""
+    import torch
+    from differentiablepointrendering_b200.device import ViewBatch
+
+    rs = [Renderer.from_scene(make_box_scene(3000, cameras=2, resolution=40, points=make_surfels(3000, 5), radiance=x),
+                              dict(ST, estimator=estimator, gradients="all")) for x in (15.0, 5.0)]
+    try:
+        batch = ViewBatch(rs, [(0, 0, 4, 0), (1, 0, 4, 0)])
+        dl = torch.full((batch.pixels, 4), 1e-4, device="cuda")
+        batch.forward_loss(None)
+        own = batch.backward(dl)
+        want = {k: (own[0][k] + own[1][k]).cpu().numpy() for k in own[0]}
+        parts = [{k: v.cpu().numpy() for k, v in g.items()} for g in own]
+        batch._gstructs[1] = batch._gstructs[0]
+        batch.forward_loss(None)
+        got = batch.backward(dl)[0]
+        torch.cuda.synchronize()
+        for k in ("opacity", "beta", "albedo", "scale", "position", "tangent_u", "tangent_v"):
+            assert min(np.linalg.norm(p[k]) for p in parts) > 0, k
+            cos, rel = _agree(got[k].cpu().numpy(), want[k])
+            assert cos >= 0.99999 and rel <= 1e-4, (k, cos, rel)
+    finally:
+        for r in rs:
+            r.close()
