@@ -694,12 +694,19 @@ void lbvh_build(const LbvhArgs& A, cudaStream_t s) {
 }
 
 namespace {
+// The bounds are moved outwards by kBoundPad of their own size before they
+// are rounded: the node test's plane distance, plane / d - o / d in one
+// multiply-add, may be off by half an ulp of o (2^-24 |o|), and a bound that
+// is a half value is not moved by the rounding.  Up to 16 times the bound's
+// distance from the origin the pad covers that; from farther away |plane - o|
+// is |o| and (plane - o) / d itself rounds as much.
+constexpr float kBoundPad = 0x1p-20f;
 __device__ __forceinline__ uint32_t pack_down(float a, float b) {
-  const __half2 h = __halves2half2(__float2half_rd(a), __float2half_rd(b));
+  const __half2 h = __halves2half2(__float2half_rd(a - kBoundPad * fabsf(a)), __float2half_rd(b - kBoundPad * fabsf(b)));
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 __device__ __forceinline__ uint32_t pack_up(float a, float b) {
-  const __half2 h = __halves2half2(__float2half_ru(a), __float2half_ru(b));
+  const __half2 h = __halves2half2(__float2half_ru(a + kBoundPad * fabsf(a)), __float2half_ru(b + kBoundPad * fabsf(b)));
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 __global__ void k_half_nodes(const BvhNode* __restrict__ in, uint32_t n, BvhNodeH* __restrict__ out) {

@@ -130,9 +130,10 @@ struct BvhNode {
 };
 static_assert(sizeof(BvhNode) == 64, "node layout");
 
-// Traversal copy of a node: the two child boxes in half precision rounded
-// outwards (lower corners down, upper corners up, so a box only grows and
-// no hit is lost) and the two child words, 32 B against BvhNode's 64 B.
+// Traversal copy of a node: the two child boxes, padded by 2^-20 of their
+// bounds, in half precision rounded outwards (lower corners down, upper
+// corners up, so a box only grows and no hit is lost) and the two child
+// words, 32 B against BvhNode's 64 B.
 //   q0 = halves (c0.lo.x c0.lo.y) (c0.hi.x c0.hi.y) (c1.lo.x c1.lo.y) (c1.hi.x c1.hi.y)
 //   q1 = halves (c0.lo.z c1.lo.z) (c0.hi.z c1.hi.z), word0, word1
 // Low and high corners sit in like words, so that one byte permutation picks

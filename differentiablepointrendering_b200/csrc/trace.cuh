@@ -164,9 +164,9 @@ struct NodeRay {
 // and whether a box is entered no farther than `best` (slab_entry and
 // entered(): in front of the origin, not past the current closest hit).  A
 // plane's distance is one multiply-add, plane / d - o / d: against (plane -
-// o) / d its rounding moves the origin by up to an ulp, far less than the
-// boxes exceed their surfels (1e-4 of the scale and 1e-3 of the normal, and
-// the rounding to half precision), so no hit is lost.
+// o) / d its rounding moves the plane by up to 2^-24 |o|, which the boxes'
+// padding covers (half_nodes): a surfel's own excess, 1e-4 of its scale, is
+// less than that for a small surfel a few units from the origin.
 __device__ __forceinline__ void node_test(const NodeRay& r, const uint4& q0, const uint4& q1, float best, float& e0,
                                           float& e1, bool& h0, bool& h1) {
   const uint32_t far_xy = r.near_xy ^ 0x4444u, far_z = r.near_z ^ 0x4444u;

@@ -45,3 +45,36 @@ def test_closest_hits_match_oracle(gpu, n, centre, size, leaf):
     assert not s.any() or np.mean(go[gp[s]] == oo[op[s]]) >= 0.9995
     hit = (gi == oi) & (gi >= 0)
     np.testing.assert_allclose(gt[hit], ot[hit], rtol=1e-5, atol=1e-6 * max(1.0, size))
+
+
+def test_hits_on_the_planes_of_boxes_away_from_the_origin(gpu):
+    # surfels whose box has an x bound that half precision holds exactly, and
+    # rays along z whose origin lies on that plane, within the box in y and z:
+    # the plane's distance is zero, and an error of o / d must not make it
+    # negative
+    h = np.arange(16.0, 64.0, 0.125, dtype=np.float32)
+    h = np.concatenate([h, -h])
+    side = np.where(np.arange(h.size) % 2 == 0, np.float32(1), np.float32(-1))
+    x = (h - side * np.float32(0.0035)).astype(np.float32)
+    s = (np.abs(h - x) * np.float32(1.00003)).astype(np.float32)
+    assert np.array_equal((x + side * (np.float32(1.0001) * s)).astype(np.float32), h)
+    n = h.size
+    y = np.linspace(-0.4, 0.4, n)
+    pts = make_surfels(n, 3)
+    pts["position"] = np.stack([x, y, np.zeros(n)], 1).astype(np.float32)
+    pts["tangent_u"] = np.tile(np.float32([[1, 0, 0]]), (n, 1))
+    pts["tangent_v"] = np.tile(np.float32([[0, 1, 0]]), (n, 1))
+    pts["scale"] = np.stack([s, np.full(n, 5e-4, np.float32)], 1)
+    scene = make_box_scene(n, points=pts)
+    st = {"photons": 64, "bounces": 1, "gather_radius": 2.0, "leaf_size": 1}
+    g, o = Renderer.from_scene(scene, st), OracleRenderer(scene, st)
+    rays = (np.stack([h, y, np.full(n, -5e-4)], 1).astype(np.float32), np.tile(np.float32([[0, 0, 1]]), (n, 1)))
+    gi, gp, gt, _, _ = g.trace_rays(*rays)
+    oi, op, ot, _, _ = o.trace_rays(*rays)
+    go, oo = g.get_point_order(), o.get_point_order()
+    g.close()
+    o.close()
+    assert np.all(oi == scene.instance_mesh.shape[0]) and np.array_equal(oo[op], np.arange(n))
+    np.testing.assert_array_equal(gi, oi)
+    np.testing.assert_array_equal(go[gp], oo[op])
+    np.testing.assert_array_equal(gt, ot)
