@@ -153,7 +153,15 @@ static_assert(sizeof(BvhNodeH) == 32, "node layout");
 #define PALE_SMEM_STACK 12
 #endif
 
+// What the walks read: the half copy, or (0) the build's own nodes.
+#ifndef PALE_HALF_NODES
+#define PALE_HALF_NODES 1
+#endif
+#if PALE_HALF_NODES
 using TravNode = BvhNodeH;
+#else
+using TravNode = BvhNode;
+#endif
 
 // Surfel arrays in BVH (leaf) order.
 struct SurfelView {

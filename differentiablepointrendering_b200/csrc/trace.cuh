@@ -111,6 +111,7 @@ __device__ __forceinline__ void surfel_eval(const SurfelView& sf, uint32_t i, V3
   x_out = x;
 }
 
+#if PALE_HALF_NODES
 // Two floats in a 64-bit register, for the packed multiply-add.
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
   unsigned long long r;
@@ -130,18 +131,6 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
 __device__ __forceinline__ unsigned long long half2_to_float2(uint32_t v) {
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
   return pack2(f.x, f.y);
-}
-
-__device__ __forceinline__ void load_node(const SceneView& S, const TravNode* __restrict__ smem_top, uint32_t idx,
-                                          uint4& q0, uint4& q1) {
-  if (idx < S.top_nodes) {
-    q0 = smem_top[idx].q0;
-    q1 = smem_top[idx].q1;
-  } else {
-    const BvhNodeH* nd = S.nodes + idx;
-    q0 = __ldg(&nd->q0);
-    q1 = __ldg(&nd->q1);
-  }
 }
 
 // A ray as the node test wants it: 1/d and -o/d by planes (x, y) and (z,
@@ -167,8 +156,9 @@ struct NodeRay {
 // o) / d its rounding moves the plane by up to 2^-24 |o|, which the boxes'
 // padding covers (half_nodes): a surfel's own excess, 1e-4 of its scale, is
 // less than that for a small surfel a few units from the origin.
-__device__ __forceinline__ void node_test(const NodeRay& r, const uint4& q0, const uint4& q1, float best, float& e0,
-                                          float& e1, bool& h0, bool& h1) {
+__device__ __forceinline__ void node_test(const NodeRay& r, const BvhNodeH& nd, float best, float& e0, float& e1,
+                                          bool& h0, bool& h1) {
+  const uint4 &q0 = nd.q0, &q1 = nd.q1;
   const uint32_t far_xy = r.near_xy ^ 0x4444u, far_z = r.near_z ^ 0x4444u;
   const float2 n0 = unpack2(fma2(half2_to_float2(__byte_perm(q0.x, q0.y, r.near_xy)), r.inv_xy, r.no_xy));
   const float2 f0 = unpack2(fma2(half2_to_float2(__byte_perm(q0.x, q0.y, far_xy)), r.inv_xy, r.no_xy));
@@ -181,6 +171,47 @@ __device__ __forceinline__ void node_test(const NodeRay& r, const uint4& q0, con
   const float x0 = fminf(fminf(fminf(f0.x, f0.y), fz.x), best), x1 = fminf(fminf(fminf(f1.x, f1.y), fz.y), best);
   h0 = fmaxf(e0, 0.0f) <= x0;
   h1 = fmaxf(e1, 0.0f) <= x1;
+}
+
+__device__ __forceinline__ uint2 child_words(const BvhNodeH& nd) { return make_uint2(nd.q1.z, nd.q1.w); }
+__device__ __forceinline__ BvhNodeH fetch_node(const BvhNodeH* nd) {
+  BvhNodeH h;
+  h.q0 = __ldg(&nd->q0);
+  h.q1 = __ldg(&nd->q1);
+  return h;
+}
+#else
+struct NodeRay {
+  V3 o, inv;
+  __device__ __forceinline__ void set(V3 o_, V3 inv_) {
+    o = o_;
+    inv = inv_;
+  }
+};
+
+__device__ __forceinline__ void node_test(const NodeRay& r, const BvhNode& nd, float best, float& e0, float& e1,
+                                          bool& h0, bool& h1) {
+  const float4 &a = nd.a, &b = nd.b, &c = nd.c;
+  e0 = slab_entry(r.o, r.inv, a.x, a.y, a.z, a.w, b.x, b.y, best);
+  e1 = slab_entry(r.o, r.inv, b.z, b.w, c.x, c.y, c.z, c.w, best);
+  h0 = entered(e0, best);
+  h1 = entered(e1, best);
+}
+
+__device__ __forceinline__ uint2 child_words(const BvhNode& nd) { return make_uint2(nd.d.x, nd.d.y); }
+__device__ __forceinline__ BvhNode fetch_node(const BvhNode* nd) {
+  BvhNode n;
+  n.a = __ldg(&nd->a);
+  n.b = __ldg(&nd->b);
+  n.c = __ldg(&nd->c);
+  n.d = __ldg(&nd->d);
+  return n;
+}
+#endif
+
+__device__ __forceinline__ TravNode load_node(const SceneView& S, const TravNode* __restrict__ smem_top,
+                                              uint32_t idx) {
+  return idx < S.top_nodes ? smem_top[idx] : fetch_node(S.nodes + idx);
 }
 
 // The traversal stack of one thread: its first PALE_SMEM_STACK entries in
@@ -292,27 +323,27 @@ struct WalkBase {
       return false;
     }
     ++visit;
-    uint4 q0, q1;
-    load_node(S, smem_top, node, q0, q1);
+    const TravNode nd = load_node(S, smem_top, node);
+    const uint2 w = child_words(nd);
     ctr.nodes++;
     float e0, e1;
     bool h0, h1;
-    node_test(ray, q0, q1, self.best, e0, e1, h0, h1);
-    h0 = h0 && q1.z != kEmptyChild;
-    h1 = h1 && q1.w != kEmptyChild;
+    node_test(ray, nd, self.best, e0, e1, h0, h1);
+    h0 = h0 && w.x != kEmptyChild;
+    h1 = h1 && w.y != kEmptyChild;
     if (h0 && h1) {
       const bool first0 = e0 <= e1;
       if (sp < kStackDepth) {
-        stk.push(sp, first0 ? q1.w : q1.z, first0 ? e1 : e0);
+        stk.push(sp, first0 ? w.y : w.x, first0 ? e1 : e0);
         ++sp;
       } else {
         flag_error(st, kErrStackOverflow);
       }
-      node = first0 ? q1.z : q1.w;
+      node = first0 ? w.x : w.y;
       return true;
     }
     if (h0 || h1) {
-      node = h0 ? q1.z : q1.w;
+      node = h0 ? w.x : w.y;
       return true;
     }
     return pop(stk, self.best);
