@@ -277,7 +277,7 @@ struct pale_handle {
   // density control scratch
   DBuf<uint32_t> dc_keys, dc_vals, dc_keys_tmp, dc_vals_tmp, dc_sort_temp, dc_flags, dc_dst, dc_list, dc_word, dc_aux;
   PointsBufs dc_points;
-  DBuf<float> query;          // inputs and outputs of the ray and lookup queries (the largest call's)
+  DBuf<float> query;          // inputs and outputs of the ray and lookup queries (QueryWords)
   HostStage stage;            // staging of large host copies
   pale_stats stats{};
   uint64_t launches_last = 0;  // kernels launched by the last render call
@@ -2264,6 +2264,27 @@ int pale_optimizer_step(pale_handle* h, const pale_optimizer* o, const pale_poin
   });
 }
 
+namespace {
+// The handle's query buffer for one call.  It is kept for the next one up to
+// 64 MB (1.2M rays), where the allocation would cost a good part of the call;
+// a larger one is given back, as the copies of such a call take longer than
+// its allocation and a scene's renders may need the memory.
+constexpr size_t kQueryKeepWords = (64u << 20) / 4;
+struct QueryWords {
+  pale_handle* h;
+  float* p;
+  QueryWords(pale_handle* h_, size_t words) : h(h_) {
+    h->query.ensure(words);
+    p = h->query.p;
+  }
+  ~QueryWords() {
+    if (h->query.n > kQueryKeepWords) h->query.free();
+  }
+  QueryWords(const QueryWords&) = delete;
+  QueryWords& operator=(const QueryWords&) = delete;
+};
+}  // namespace
+
 int pale_trace_rays(pale_handle* h, uint32_t n, const float* o, const float* d, int32_t* inst, int32_t* prim,
                     float* t, float* alpha, float* pos) {
   if (!h) return PALE_ERR_ARGUMENT;
@@ -2273,8 +2294,8 @@ int pale_trace_rays(pale_handle* h, uint32_t n, const float* o, const float* d, 
     use_stream(h, h->own_stream);
     cudaStream_t s = h->stream;
     // inputs and outputs in the handle's query buffer: 6 and 7 words a ray
-    h->query.ensure(13ull * n);
-    float *dO = h->query.p, *dD = dO + 3ull * n, *dP = dD + 3ull * n, *dT = dP + 3ull * n, *dA = dT + n;
+    const QueryWords q(h, 13ull * n);
+    float *dO = q.p, *dD = dO + 3ull * n, *dP = dD + 3ull * n, *dT = dP + 3ull * n, *dA = dT + n;
     int32_t *dI = reinterpret_cast<int32_t*>(dA + n), *dR = dI + n;
     copy_in(h, {DeviceIn{dO, o, 12ull * n}, DeviceIn{dD, d, 12ull * n}}, false);
     CK(cudaMemsetAsync(h->run.p, 0, sizeof(RunState), s));
@@ -2297,8 +2318,8 @@ int pale_trace_transmittance(pale_handle* h, uint32_t n, const float* o, const f
     if (!n) return PALE_OK;
     use_stream(h, h->own_stream);
     cudaStream_t s = h->stream;
-    h->query.ensure(9ull * n);
-    float *dO = h->query.p, *dD = dO + 3ull * n, *dT = dD + 3ull * n, *dX = dT + n;
+    const QueryWords q(h, 9ull * n);
+    float *dO = q.p, *dD = dO + 3ull * n, *dT = dD + 3ull * n, *dX = dT + n;
     int32_t* dI = reinterpret_cast<int32_t*>(dX + n);
     copy_in(h, {DeviceIn{dO, o, 12ull * n}, DeviceIn{dD, d, 12ull * n}}, false);
     CK(cudaMemsetAsync(h->run.p, 0, sizeof(RunState), s));
@@ -2319,8 +2340,8 @@ int pale_gather_irradiance(pale_handle* h, uint32_t n, const float* pts, const f
     if (!n) return PALE_OK;
     use_stream(h, h->own_stream);
     cudaStream_t s = h->stream;
-    h->query.ensure(9ull * n);
-    float *dP = h->query.p, *dN = dP + 3ull * n, *dE = dN + 3ull * n;
+    const QueryWords q(h, 9ull * n);
+    float *dP = q.p, *dN = dP + 3ull * n, *dE = dN + 3ull * n;
     copy_in(h, {DeviceIn{dP, pts, 12ull * n}, DeviceIn{dN, nrm, 12ull * n}}, false);
     gather_points(h->view(), n, dP, dN, dE, s);
     CK(cudaGetLastError());

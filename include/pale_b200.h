@@ -502,7 +502,10 @@ int pale_densify_long_axis_split(pale_handle *h, const float *d_importance,
 /* Closest-hit queries against the scene (intersectScene in FirstHit mode,
  * IntersectionKernels.h:954-1097).  Host arrays of n rays; outputs:
  * instance (-1 = miss), primitive (surfel in BVH order or triangle id),
- * world t, alpha_geom, hit position (n*3). */
+ * world t, alpha_geom, hit position (n*3).  The handle keeps the device
+ * buffer of its queries (52 bytes per ray, 36 per transmittance ray or
+ * lookup) until it is destroyed, up to 64 MB; a larger query's is freed
+ * when it returns. */
 int pale_trace_rays(pale_handle *h, uint32_t n, const float *origins,
                     const float *directions, int32_t *instance,
                     int32_t *primitive, float *t, float *alpha_geom,
