@@ -495,10 +495,12 @@ void size_wavefronts(pale_handle* h, uint64_t all_pix, uint32_t max_pix) {
   }
   const uint64_t want = all_pix * std::max<uint32_t>(1u, st.gather_passes);
   const uint64_t cg_limit = st.gather_batch_paths ? st.gather_batch_paths : (1ull << 25);
-  // (2^28 at most: a round's records stay below 2^31, the mark of the heavy
-  // lookups; a view is below 2^24 pixels, so a pass of it always fits)
+  // (a round's records, kGatherHits per path, stay within 2^31, whose bit
+  // marks the heavy lookups; a view is below 2^24 pixels, so a pass of it
+  // always fits)
+  static_assert(kGatherHits <= 1 << 7, "a pass of a view of 2^24 pixels");
   const uint32_t path_cap = (uint32_t)std::min<uint64_t>(
-      std::max<uint64_t>(std::max<uint64_t>(all_pix, 1), std::min<uint64_t>(want, cg_limit)), 1ull << 28);
+      std::max<uint64_t>(std::max<uint64_t>(all_pix, 1), std::min<uint64_t>(want, cg_limit)), (1ull << 31) / kGatherHits);
   if (path_cap > h->path_cap) {
     h->path_cap = path_cap;
     h->cg_paths.alloc(h->path_cap); h->cg_paths2.alloc(h->path_cap);

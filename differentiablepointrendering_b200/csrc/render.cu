@@ -1174,8 +1174,8 @@ __device__ __forceinline__ bool event_looks_up(const uint4& d) {
 // ms, the heavy ones alike).
 constexpr uint32_t kSortEntries = 32768;
 
-// Marks a lookup of the order as left to the heavy lookups (lookups are
-// below 2^28).
+// Marks a lookup of the order as left to the heavy lookups (a lookup's number
+// is below 2^31: the path capacity times kGatherHits).
 constexpr uint32_t kHeavyMark = 0x80000000u;
 
 // The radiance a layer adds to its path: Lo * weight.

@@ -1079,6 +1079,8 @@ __device__ __forceinline__ bool window_lit(const GridView& G, V3 x) {
 #define PALE_LOOKUP_HEAVY 256
 #endif
 constexpr uint32_t kLookupHeavy = PALE_LOOKUP_HEAVY;
+static_assert(PALE_LOOKUP_HEAVY >= 32 && PALE_LOOKUP_HEAVY % 32 == 0 && PALE_LOOKUP_HEAVY < 4095,
+              "PALE_LOOKUP_HEAVY: whole words of 32 photons, below the row length that counts as heavy");
 
 // Shared memory of a group's lookup: per non-empty row its first photon less
 // its place in the sequence; a bit per photon of the sequence, set where a
@@ -1277,6 +1279,7 @@ __device__ __forceinline__ V3 gather_irradiance_lanes(const GridView& G, const G
 #define PALE_LOOKUP_LANES 8
 #endif
 constexpr int kLookupLanes = PALE_LOOKUP_LANES;
-constexpr int kLookupGroups = 32 / kLookupLanes;   // queries of a warp at a time
+static_assert(kLookupLanes == 4 || kLookupLanes == 8 || kLookupLanes == 16,
+              "PALE_LOOKUP_LANES: 4, 8 or 16 lanes (the 16 squared distances are split over them)");
 
 }  // namespace pale

@@ -21,3 +21,15 @@ def _compile(tmp_path, body, *flags):
 def test_half_nodes_selects_the_traversal_nodes(tmp_path, half, size):
     r = _compile(tmp_path, f'static_assert(sizeof(pale::TravNode) == {size}, "node");\n', f"-DPALE_HALF_NODES={half}")
     assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("knob,good,bad", [("PALE_LOOKUP_HEAVY", (32, 96, 512), (16, 100, 4096)),
+                                           ("PALE_LOOKUP_LANES", (4, 16), (2, 12, 32))])
+def test_lookup_knobs_are_guarded(tmp_path, knob, good, bad):
+    # other values would write past the group's shared memory or leave parts of it unwritten
+    for v in good:
+        r = _compile(tmp_path, "", f"-D{knob}={v}")
+        assert r.returncode == 0, r.stderr
+    for v in bad:
+        r = _compile(tmp_path, "", f"-D{knob}={v}")
+        assert r.returncode != 0 and knob in r.stderr, v
