@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(1024) k_queue_scan(RunState* st, const uint2* 
 
 // Compacts staged rays (and photon deposits) of the `n_in` input slots,
 // and takes the rays into their bins for the next bounce's walk.
-__device__ __forceinline__ void place_side(const PhotonArgs& A, uint32_t slot, uint32_t rank) {
+__device__ __forceinline__ void place_deposit(const PhotonArgs& A, uint32_t slot, uint32_t rank) {
   const uint64_t dst = (uint64_t)A.st->photon_base + rank;
   if (dst < A.ps.capacity) {
     A.ps.a[dst] = A.ps.sa[slot];
@@ -269,7 +269,6 @@ __device__ __forceinline__ void place_side(const PhotonArgs& A, uint32_t slot, u
     A.ps.c[dst] = A.ps.sc[slot];
   }
 }
-__device__ __forceinline__ void place_side(const AdjointArgs&, uint32_t, uint32_t) {}
 
 template <class Args>   // PhotonArgs, AdjointArgs
 __global__ void k_queue_scatter(Args A, uint32_t parity, int emission, uint32_t emission_n) {
@@ -307,7 +306,9 @@ __global__ void k_queue_scatter(Args A, uint32_t parity, int emission, uint32_t 
     const uint32_t rank = bin_rank(A.rb.bins, bin);
     if (bin != kInvalid) A.rb.at[dst] = make_uint2(bin, rank);
   }
-  if (side) place_side(A, slot, off.y + rs);
+  if constexpr (std::is_same<Args, PhotonArgs>::value) {
+    if (side) place_deposit(A, slot, off.y + rs);
+  }
 }
 
 __global__ void k_advance(RunState* st, uint32_t by) {
@@ -1194,6 +1195,7 @@ __device__ __forceinline__ float4 layer_radiance(const SceneView& S, uint32_t ki
 // The lookups of a gather round: a record's point, normal and index word; a
 // lookup's result is the layer's contribution, over the record's first float4.
 struct RoundLookups {
+  static constexpr bool kMayBeFew = true;   // below kSortEntries
   FrameArgs A;
   uint32_t round;
   struct Keep {
@@ -1231,6 +1233,7 @@ struct RoundLookups {
 // The lookups of a bounce's events (k_transport's): the event's point and
 // normal; a lookup's irradiance takes the normal's place.
 struct EventLookups {
+  static constexpr bool kMayBeFew = false;   // kSplitPaths or more
   AdjointArgs A;
   using Keep = float;
   __device__ __forceinline__ const SceneTable& scenes() const { return A.scenes; }
@@ -1431,13 +1434,15 @@ static void run_lookups(const Lookups& Q, RunState* st, LookupOrder so, uint64_t
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lookup<Lookups, kMulti>, kBlock, 0);
   const uint32_t grid = std::min<uint32_t>((uint32_t)sms * 8u, blocks_for(items));
-  if (entries >= kSortEntries) {
+  bool sort = true;
+  if constexpr (Lookups::kMayBeFew) sort = entries >= kSortEntries;
+  if (sort) {
     so.mask = gather_bins(entries) - 1u;
     cudaMemsetAsync(so.bins, 0, ((size_t)so.mask + 1) * sizeof(uint32_t), s);
     k_lookup_lit<Lookups, kMulti, true><<<grid, kBlock, 0, s>>>(Q, so); note_launch();
     k_bin_offsets<<<(so.mask + 1u) / (kBlock * kBinItems), kBlock, 0, s>>>(so.bins, &st->lookup_next); note_launch();
     k_lookup_order<<<grid, kBlock, 0, s>>>(Q, so); note_launch();
-  } else {
+  } else if constexpr (Lookups::kMayBeFew) {
     k_lookup_lit<Lookups, kMulti, false><<<grid, kBlock, 0, s>>>(Q, so); note_launch();
   }
   k_lookup<Lookups, kMulti><<<(uint32_t)std::max(1, sms * std::max(1, per_sm)), kBlock, 0, s>>>(Q, so); note_launch();
@@ -2447,6 +2452,7 @@ void adjoint_raygen(const AdjointArgs& a, uint32_t npaths, cudaStream_t s) {
 // paths over dense photons, 0.32 against 0.32 ms of 262k paths over sparse
 // ones.
 constexpr uint32_t kSplitPaths = 131072u;
+static_assert(kSplitPaths >= kSortEntries, "EventLookups::kMayBeFew");
 // One bounce of every job of the batch; npaths bounds the live queue.
 void adjoint_bounce(AdjointArgs a, uint32_t bounce, bool last, uint32_t npaths, cudaStream_t s) {
   const uint32_t nb = blocks_for(npaths);
