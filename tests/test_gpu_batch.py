@@ -168,3 +168,48 @@ def test_entries_that_share_gradient_arrays_hold_the_sum(gpu, estimator):
     finally:
         for r in rs:
             r.close()
+
+
+def _alone_equals(batch, grads, dl, groups):
+    """The batch's per-scene gradients against each scene's views in a call of their own."""
+    import torch
+    from differentiablepointrendering_b200.device import ViewBatch
+
+    for k, r in enumerate(batch.renderers):
+        mine = [i for i, v in enumerate(batch.views) if v[0] == k]
+        offs = np.concatenate([[0], np.cumsum([w * h for w, h in batch.sizes])])
+        own = ViewBatch([r], [(0,) + batch.views[i][1:4] for i in mine])
+        own.forward_loss(None, trace_photons=False)   # what the gather estimator differentiates
+        g1 = own.backward(torch.cat([dl[offs[i]:offs[i + 1]] for i in mine]).contiguous())[0]
+        torch.cuda.synchronize()
+        for key in groups:
+            a, b = grads[k][key], g1[key].cpu().numpy()
+            assert np.linalg.norm(b) > 0, (k, key)
+            cos, rel = _agree(a, b)
+            assert cos >= 0.99999 and rel <= 1e-4, (k, key, cos, rel)
+
+
+@pytest.mark.parametrize("estimator,res", [("reference", 200), ("gather", 64)])
+def test_all_groups_of_two_scenes_equal_each_alone(gpu, estimator, res):
+    """Two scenes with photon maps of their own, every gradient group.
+    reference: 160,000 adjoint paths, whose events are looked up before the
+    transport (each scene alone has 80,000 and looks them up inside it), some
+    of them over hundreds of photons; gather: the sweep's terms of a second
+    scene."""
+    import torch
+    from differentiablepointrendering_b200.device import ViewBatch
+
+    st = dict(ST, photons=100000, adjoint_passes=2, gather_passes=2, estimator=estimator, gradients="all")
+    rs = [Renderer.from_scene(make_box_scene(n, cameras=2, resolution=res, points=make_surfels(n, s), radiance=x),
+                              dict(st, seed=s)) for n, s, x in ((4000, 11, 15.0), (6000, 22, 6.0))]
+    try:
+        batch = ViewBatch(rs, [(1, 0, 2, 0), (0, 0, 2, 0)])
+        batch.forward_loss(None)
+        dl = torch.zeros(batch.pixels, 4, device="cuda")
+        dl[:, :3] = (batch.raw[:, :3] - 0.3) / batch.pixels
+        grads = [{k: v.cpu().numpy() for k, v in g.items()} for g in batch.backward(dl)]
+        torch.cuda.synchronize()
+        _alone_equals(batch, grads, dl, ("opacity", "beta", "albedo", "scale", "position", "tangent_u", "tangent_v"))
+    finally:
+        for r in rs:
+            r.close()

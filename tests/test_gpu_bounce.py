@@ -54,7 +54,9 @@ def test_adjoint_matches_oracle(gpu, res, gradients):
     gg, _ = g.render_backward(dl)
     go, _ = o.render_backward(dl)
     assert abs(g.stats()["gradient_events"] - o.stats()["gradient_events"]) <= 1e-2 * o.stats()["gradient_events"] + 2
-    for k in ("opacity",) if gradients == "opacity" else ("opacity", "albedo", "beta"):
+    groups = ("opacity",) if gradients == "opacity" else ("opacity", "beta", "albedo", "scale", "position", "tangent_u",
+                                                          "tangent_v")
+    for k in groups:
         a, b = np.empty_like(gg[k]), np.empty_like(go[k])
         a[g.get_point_order()] = gg[k]
         b[o.get_point_order()] = go[k]
