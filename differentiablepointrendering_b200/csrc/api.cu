@@ -465,10 +465,11 @@ void size_queues(pale_handle* h, size_t n) {
 // The wavefront buffers of camera-gather and adjoint calls whose views hold
 // all_pix pixels, the largest view max_pix (grown, never shrunk):
 // - adjoint: the (view, pass) jobs of a call trace together, up to 2^24
-//   paths per batch (about 5.4 GB of queues and events), or the
-//   adjoint_batch_paths setting;
+//   paths per batch (330 bytes a path: 5.5 GB of queues, events and walk
+//   records; 32 more with every gradient group), or the adjoint_batch_paths
+//   setting;
 // - camera gather: every pass of every pixel in flight when that fits in
-//   2^25 paths (3.2 GB of path queues, 8.6 GB of lookup records, 1 GB of
+//   2^25 paths (3.2 GB of path queues, 8.6 GB of lookup records, 4.8 GB of
 //   per-entry state), or the gather_batch_paths setting, else chunks of
 //   whole passes; at least every pixel once.
 void size_wavefronts(pale_handle* h, uint64_t all_pix, uint32_t max_pix) {
@@ -1439,10 +1440,11 @@ struct DeviceIn {
 // A staged copy's place in the stage.
 size_t stage_slot(size_t bytes) { return (bytes + 255) & ~size_t(255); }
 
-// Whether `total` bytes go through the stage.  With grow, the stage is made
-// as large; a query (rays, lookups) uses the stage that renders have left and
-// allocates none: pinning memory costs more than its copies save (14 MB, 10
-// ms), and a caller's first query counts.
+// Whether `total` bytes go through the stage.  With grow (renders and
+// parameter reads, which loops repeat), the stage is made as large, and the
+// first such call pays for it: pinning memory costs more than one call's
+// copies save (14 MB, 10 ms).  A query (rays, lookups), often a program's only
+// one, uses the stage that renders have left and allocates none.
 bool use_stage(pale_handle* h, size_t total, bool grow) {
   if (total < kStageMinBytes) return false;
   return grow ? h->stage.ensure(total, h->stream) : h->stage.p && h->stage.n >= total;

@@ -145,10 +145,12 @@ struct BvhNodeH {
 };
 static_assert(sizeof(BvhNodeH) == 32, "node layout");
 // Traversal stack entries per thread kept in shared memory (the rest local,
-// whose loads and stores go through L1).  Closest hits at 8, 12, 14 and 16
-// entries: 79.1, 76.3, 76.0 and 76.1 ms on 200k surfels x 8 views; the 8-hit
-// walk 56.8, 55.9, 57.0 and 57.0 ms (its hits take 16 KB a block as well, so
-// past 12 its L1 gets too small).
+// whose loads and stores go through L1).  A step of 200k surfels x 8 views at
+// 8, 10, 12 and 14 entries: 261.2, 259.1, 258.3 and 259.5 ms, its camera rounds
+// 69.8, 69.1, 69.0 and 70.3; those of three scenes in one call 18.6, 18.7, 18.7
+// and 20.5 ms.  The 8-hit walk's block takes 16 KB of hits and, with several
+// scenes, 16 KB of staged nodes beside 24 KB of stack: four blocks fill the
+// SM's 228 KB (28 KB of L1 left), and from 13 entries on only three fit.
 #ifndef PALE_SMEM_STACK
 #define PALE_SMEM_STACK 12
 #endif

@@ -153,8 +153,14 @@ __device__ __forceinline__ uint32_t ray_bin(const AdjointArgs& A, const RayRec& 
   return ray_bin(A.scenes.s[sid].grid, ry, sid, multi, A.rb.log2);
 }
 
-// Enough bins that a bin holds a few rays, at most 4 MB of counters; below
-// 16k rays the walk is shorter than the grouping.
+// Enough bins that a bin holds a few rays, at most 4 MB of counters.  Grouping
+// costs a clear, a launch and scattered records, 6-10 us a bounce below 65k
+// rays, and about repays itself above: six bounces with and without it 0.54
+// and 0.49 ms for 4k rays of 1k surfels, 0.91 and 0.88 for 16k of 10k surfels,
+// 1.21 and 1.16 for 65k, 7.21 and 7.19 for 2M; 2M of 1k surfels 4.32 and 4.41;
+// 16M of 200k surfels 89.9 and 90.7 for the traced bounces, 111.6 and 111.5 with
+// the rest of the adjoint; 1M photons among 200k surfels 5.0 and 4.9.  The line
+// keeps it from the queues where it costs the largest share.
 int ray_bins_log2(uint32_t rays) {
   if (rays < PALE_RAY_BIN_MIN) return 0;
   int b = 11;
@@ -2447,10 +2453,13 @@ void adjoint_raygen(const AdjointArgs& a, uint32_t npaths, cudaStream_t s) {
 
 // Paths of a batch from which its events' lookups are taken out of the
 // transport, into the kernels of the camera's lookups: their launches cost
-// about 20 us a bounce, the lookups inside the transport 27 ms of a step of
-// 200k surfels x 8 views against 17 ms outside, 5.2 against 3.1 ms of 393k
-// paths over dense photons, 0.32 against 0.32 ms of 262k paths over sparse
-// ones.
+// about 30 us a bounce, and what they save grows with the photons of a lookup.
+// Adjoint with the lookups inside and outside: 65k paths over dense photons
+// (1M, 20k surfels) 3.03 and 2.69 ms, 131k 4.12 and 3.20, 524k 9.86 and 5.94;
+// over sparse ones (100k, 10k surfels) 1.26 and 1.45, 1.50 and 1.69, 3.01 and
+// 3.00; 200k surfels with 1M photons 1.89 and 2.08, 2.21 and 2.35, 3.68 and
+// 3.65; the 16.8M paths of 8 views 27 and 17 ms for lookups and transport.  At
+// the line the dense case gains 0.9 ms where the sparse ones lose 0.15.
 constexpr uint32_t kSplitPaths = 131072u;
 static_assert(kSplitPaths >= kSortEntries, "EventLookups::kMayBeFew");
 // One bounce of every job of the batch; npaths bounds the live queue.

@@ -1070,11 +1070,12 @@ __device__ __forceinline__ bool window_lit(const GridView& G, V3 x) {
 // stand in shared memory), so that short rows leave no lane idle: on lookups
 // of up to 256 photons about 190 warp instructions a lookup against 380 by a
 // whole warp.  The photon numbers of neighbouring queries are neighbours when
-// the queries are grouped by cell (L1 hits 52 -> 77%).  A query of more than
+// the queries are grouped by cell.  A query of more than
 // kLookupHeavy photons is not done (heavy; its result is undefined): there
 // the photons' own work counts, which a whole warp shares better.
-// (128, 256 and 512 measured 77, 73 and 73 ms of lookups on 200k surfels, 8
-// views; 1.61, 1.50 and 1.56 ms on six small ones)
+// (128, 256 and 512: 74.3, 68.6 and 66.1 ms of camera lookups on 200k surfels,
+// 8 views; 18.8, 17.4 and 17.1 ms on three scenes; 1.51, 1.35 and 1.47 ms on
+// six small views)
 #ifndef PALE_LOOKUP_HEAVY
 #define PALE_LOOKUP_HEAVY 256
 #endif
@@ -1124,7 +1125,9 @@ __device__ __forceinline__ V3 gather_irradiance_lanes(const GridView& G, const G
   const float inv_cx = GC.inv_cx;
   const uint32_t total_ph = GC.total_ph;
   const float reach2 = r2 * 1.002f;
-  // squared distances of x to the window's y rows (0..7) and z slabs (8..15)
+  // squared distances of x to the window's y rows (0..7) and z slabs (8..15);
+  // a window that rounding made wider than 8 cells has its photons within r
+  // in the first 8 (there a cell is finer than the positions)
 #pragma unroll
   for (int t = 0; t < 16 / kLanes; ++t) {
     const int i = p + t * kLanes;
@@ -1273,8 +1276,9 @@ __device__ __forceinline__ V3 gather_irradiance_lanes(const GridView& G, const G
   return v3(ax[0] * s, ay[0] * s, az[0] * s);
 }
 
-// Lanes per short lookup: 4, 8 and 16 measured 72, 73 and 82 ms on 200k
-// surfels, 8 views, and 1.78, 1.50 and 1.40 ms on six small ones.
+// Lanes per short lookup: 4, 8 and 16 measured 67.1, 68.6 and 75.6 ms of camera
+// lookups on 200k surfels, 8 views; 16.6, 17.4 and 18.0 ms on three scenes;
+// 1.44, 1.35 and 1.31 ms on six small views.
 #ifndef PALE_LOOKUP_LANES
 #define PALE_LOOKUP_LANES 8
 #endif

@@ -99,7 +99,9 @@ typedef struct pale_handle pale_handle;
  * camera paths again with the forward's seeds (deterministic, so the
  * layers are the forward's) into a scratch store of one chunk; AUTO
  * checkpoints while the store fits vertex_store_bytes (0: half the free
- * device memory) and replays the chunks that do not fit. */
+ * device memory) and replays the chunks that do not fit.  A GATHER backward
+ * with all gradient groups also holds 64 bytes per surfel of the call's
+ * scenes, in the handle of scenes[0] until it is destroyed. */
 #define PALE_VERTICES_AUTO 0u
 #define PALE_VERTICES_CHECKPOINT 1u
 #define PALE_VERTICES_REPLAY 2u
