@@ -123,13 +123,14 @@ class ClockSampler:
 # Algorithmic bytes per kernel of one step, from the device counters:
 # a ray segment reads/writes 32 + 32 B of ray state and a 16 B hit record,
 # 32 B per BVH node visited and 52 B per surfel test; a photon lookup reads
-# 36 B per photon scanned and 8 B (two cell offsets) per grid row of its
-# window (25 rows); the adjoint bounce also reads and writes its 48 B
-# pending state, and its three kernels (mesh pass, persistent walk,
-# shading) pass 128 B of hit and walk records per ray between them (two 32 B
-# records, each written and read); a gradient event is a 64 B record, its lookup and
-# an 8 B atomic read-modify-write.
-ROWS_PER_QUERY = 25
+# a 4 B word of the grid's occupancy and 36 B per photon scanned (not counted:
+# the offsets of its rows, since most lookups end at the word); the adjoint
+# bounce also reads and writes its 48 B pending state, and its three kernels
+# (mesh pass, persistent walk, shading) pass 128 B of hit and walk records per
+# ray between them (two 32 B records, each written and read); a listed
+# gradient event (each has one lookup) is a 64 B record and an 8 B atomic
+# read-modify-write.  Nodes, surfels and photons come from L1 and L2 for the
+# most part, so the rate of these bytes is no fraction of the HBM's.
 FWD_COUNTERS = ("photon_segments", "photons_stored", "gather_segments", "gather_node_visits", "gather_surfel_tests",
                 "gather_queries", "gather_photons_scanned")
 ADJ_COUNTERS = ("adjoint_segments", "node_visits", "surfel_tests", "gradient_events", "gather_queries",
@@ -138,7 +139,7 @@ ADJ_COUNTERS = ("adjoint_segments", "node_visits", "surfel_tests", "gradient_eve
 
 def kernel_bytes(sf: dict, sb: dict, estimator: str = "reference", all_grads: bool = False) -> dict:
     seg = lambda segs, nodes, tests: 80.0 * segs + 32.0 * nodes + 52.0 * tests
-    look = lambda q, scanned: 36.0 * scanned + 8.0 * ROWS_PER_QUERY * q
+    look = lambda q, scanned: 36.0 * scanned + 4.0 * q
     fwd_q = sf["gather_queries"]
     adj_q = sb["gather_queries"]
     out = {
@@ -155,7 +156,7 @@ def kernel_bytes(sf: dict, sb: dict, estimator: str = "reference", all_grads: bo
         return out
     out["k_adj_bounce"] = seg(sb["adjoint_segments"], sb["node_visits"], sb["surfel_tests"]) \
         + (96.0 + 128.0) * sb["adjoint_segments"]
-    out["k_transport"] = 72.0 * sb["gradient_events"] + look(adj_q, sb["photons_scanned"])
+    out["k_transport"] = 72.0 * adj_q + look(adj_q, sb["photons_scanned"])
     return out
 
 
@@ -177,16 +178,20 @@ def read_peaks():
         return None
 
 
-def read_traffic(kernel: str, launch_ms: float):
-    """DRAM bytes of one launch of `kernel`: the DRAM rate of its ncu
-    capture on the small case (profiles/traffic.json) times the launch's
-    live device time; None without a capture."""
-    p = os.path.join(ROOT, "profiles", "traffic.json")
+def read_capture(kernel: str, key: str):
+    """A figure of the kernel's ncu capture on the small case
+    (profiles/traffic.json); None without one."""
     try:
-        rate = json.load(open(p))[kernel]["dram_bytes_per_s"]
+        return json.load(open(os.path.join(ROOT, "profiles", "traffic.json")))[kernel][key]
     except Exception:
         return None
-    return int(rate * launch_ms / 1e3)
+
+
+def read_traffic(kernel: str, launch_ms: float):
+    """DRAM bytes of one launch of `kernel`: the DRAM rate of its ncu
+    capture times the launch's live device time; None without a capture."""
+    rate = read_capture(kernel, "dram_bytes_per_s")
+    return None if rate is None else int(rate * launch_ms / 1e3)
 
 
 def cpu_reference_run(w: dict, steps: int = 1, warmup: int = 0):
@@ -602,20 +607,24 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         extra["c4"] = c4_measure(dev, tune=not args.no_tune)
     peaks = read_peaks()
     hbm = peaks["hbm_gbs"] if peaks else 6650.0
-    # per-kernel device time (events around every launch, stats step) and
-    # algorithmic bytes; the roofline entry is the kernel with the most time
+    # per-kernel device time (events around every launch, stats step),
+    # algorithmic bytes and DRAM traffic; the roofline entry is the kernel
+    # with the most time: its DRAM rate against the HBM's and, since that is
+    # far from its peak, the unit that is busiest
     kb = kernel_bytes(sf, sb, args.estimator, args.gradients == "all")
     kt = kernel_times(sf, sb, args.estimator)
     kernels = {}
     for k in kb:
         ms, n = kt[k]
         n = max(1, int(n))
-        ach = kb[k] / (ms / 1e3) / 1e9 if ms > 0 else 0.0
+        dram = read_capture(k, "dram_bytes_per_s")
         kernels[k] = {"ms_per_step": round(ms, 3), "launches": n, "launch_ms": round(ms / n, 4),
-                      "algorithmic_bytes_per_launch": int(kb[k] / n), "achieved_gbs": round(ach, 1),
-                      "frac": round(ach / hbm, 4), "dram_bytes_per_launch": read_traffic(k, ms / n)}
+                      "algorithmic_bytes_per_launch": int(kb[k] / n),
+                      "algorithmic_gbs": round(kb[k] / (ms / 1e3) / 1e9, 1) if ms > 0 else 0.0,
+                      "dram_bytes_per_launch": read_traffic(k, ms / n),
+                      "dram_frac": None if dram is None else round(dram / 1e9 / hbm, 4)}
     top = max(kernels, key=lambda k: kernels[k]["ms_per_step"])
-    achieved = kernels[top]["achieved_gbs"]
+    dram, busiest = read_capture(top, "dram_bytes_per_s"), read_capture(top, "busiest") or [None, None]
     traffic = read_traffic(top, kernels[top]["launch_ms"])
     if args.skip_cpu:
         cpu_val, cpu_desc, cpu_kind = None, "skipped", None
@@ -632,10 +641,12 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         "e2e": {"value": round(e2e_value, 3), "unit": "Mrays/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "steps": e2e_steps, "warmup": 1},
         "gpu_launches": launches * args.steps,
-        "roofline": {"kernel": top, "bound": "hbm", "achieved": round(achieved, 1),
-                     "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4),
+        "roofline": {"kernel": top, "bound": busiest[0], "busiest_pct": busiest[1],
+                     "achieved": None if dram is None else round(dram / 1e9, 1),
+                     "peak": hbm, "unit": "GB/s", "frac": kernels[top]["dram_frac"],
                      "traffic": traffic, "peak_source": "measured" if peaks else "fallback",
                      "algorithmic_bytes_per_launch": kernels[top]["algorithmic_bytes_per_launch"],
+                     "algorithmic_gbs": kernels[top]["algorithmic_gbs"],
                      "launch_ms": kernels[top]["launch_ms"], "launches_per_step": kernels[top]["launches"]},
         "kernels": kernels,
         "cpu_baseline": {"value": round(cpu_val, 4) if cpu_val else None, "unit": "Mrays/s",

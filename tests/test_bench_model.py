@@ -1,7 +1,8 @@
 """The bench's measurement model on CPU: the algorithmic bytes per kernel
 follow the per-unit figures (ray segment 80 B + 32 B per node + 52 B per
-surfel test; lookup 36 B per photon + 8 B per window row; the adjoint
-bounce's pending state and inter-kernel records; 72 B per gradient event),
+surfel test; lookup 36 B per photon + a 4 B occupancy word; the adjoint
+bounce's pending state and inter-kernel records; 72 B per listed gradient
+event, which are those that look photons up),
 every timed kernel group has a DRAM traffic entry for the roofline, and
 the counters the bench line reports are the ones the model reads."""
 import json
@@ -27,11 +28,10 @@ def _counters():
 def test_algorithmic_bytes_follow_the_unit_figures():
     sf, sb = _counters()
     kb = bench.kernel_bytes(sf, sb)
-    rows = bench.ROWS_PER_QUERY
     assert kb["k_cg_round"] == 80 * 1000 + 32 * 30000 + 52 * 5000
-    assert kb["k_cg_lookup"] == 36 * 45000 + 8 * rows * 900
+    assert kb["k_cg_lookup"] == 36 * 45000 + 4 * 900
     assert kb["k_adj_bounce"] == 80 * 700 + 32 * 20000 + 52 * 3000 + (96 + 128) * 700
-    assert kb["k_transport"] == 72 * 300 + 36 * 7000 + 8 * rows * 200
+    assert kb["k_transport"] == 72 * 200 + 36 * 7000 + 4 * 200
 
 
 def test_every_timed_kernel_has_traffic_and_counters():
@@ -40,6 +40,7 @@ def test_every_timed_kernel_has_traffic_and_counters():
     with open(os.path.join(os.path.dirname(HERE), "profiles", "traffic.json")) as f:
         traffic = json.load(f)
     assert timed <= set(traffic), timed - set(traffic)
+    assert all(bench.read_capture(k, "busiest")[1] > 0 for k in timed)
     rates = {k: v["dram_bytes_per_s"] for k, v in traffic.items() if not k.startswith("_")}
     assert all(isinstance(v, int) and v > 0 for v in rates.values())
     for k in timed:
