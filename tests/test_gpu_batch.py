@@ -213,3 +213,36 @@ def test_all_groups_of_two_scenes_equal_each_alone(gpu, estimator, res):
     finally:
         for r in rs:
             r.close()
+
+
+@pytest.mark.parametrize("block", [64, 128])
+def test_walk_blocks_give_the_same_images(gpu, block):
+    """The walks (photons, camera layers, adjoint) with blocks of 64 and 128
+    threads against 256, one scene alone and two together."""
+    import torch
+    from differentiablepointrendering_b200.device import ViewBatch
+
+    scenes = [_scene(3000, 1, 64, 7), _scene(5000, 1, 96, 8)]
+    views = [(0, 0, 4, 0), (1, 0, 2, 0)]
+    out = []
+    for b in (256, block):
+        rs = [Renderer.from_scene(sc, dict(ST, walk_block=b)) for sc in scenes]
+        try:
+            alone, both = ViewBatch(rs[:1], views[:1]), ViewBatch(rs, views)
+            res = []
+            for batch in (alone, both):
+                batch.forward_loss(None)
+                dl = torch.zeros(batch.pixels, 4, device="cuda")
+                dl[:, :3] = (batch.raw[:, :3] - 0.3) / batch.pixels
+                g = batch.backward(dl)
+                torch.cuda.synchronize()
+                res.append((batch.raw.cpu().numpy().copy(), [x["opacity"].cpu().numpy().copy() for x in g]))
+            out.append(res)
+        finally:
+            for r in rs:
+                r.close()
+    for (raw0, g0), (raw1, g1) in zip(*out):
+        np.testing.assert_array_equal(raw0, raw1)
+        for a, b in zip(g1, g0):
+            cos, rel = _agree(a, b)
+            assert cos >= 0.99999 and rel <= 1e-4, (cos, rel)

@@ -2,6 +2,8 @@
 directions and positions where the node test could lose one: axis-parallel
 and nearly parallel rays, negative zeros, every octant, clouds away from the
 origin and of another size, few surfels and leaves of several."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -78,3 +80,32 @@ def test_hits_on_the_planes_of_boxes_away_from_the_origin(gpu):
     np.testing.assert_array_equal(gi, oi)
     np.testing.assert_array_equal(go[gp], oo[op])
     np.testing.assert_array_equal(gt, ot)
+
+
+@pytest.mark.parametrize("instances", [31, 32, 33, 65, 100])
+def test_meshes_of_many_instances_match_oracle(gpu, instances):
+    # instances are taken 32 at a time: boxes first, then each ray its own
+    rng = np.random.default_rng(instances)
+    scene = make_box_scene(200, points=make_surfels(200, 3))
+    m = np.tile(np.eye(4), (instances, 1, 1))
+    for k in range(instances):
+        q = np.linalg.qr(rng.normal(size=(3, 3)))[0]
+        m[k, :3, :3] = q * rng.uniform(0.02, 0.3)
+        m[k, :3, 3] = rng.uniform(-0.5, 0.5, 3)
+    m[-1] = scene.object_to_world[-1]                      # the light
+    first = [0] * (instances - 1)
+    scene = dataclasses.replace(
+        scene, instance_mesh=np.asarray(first + [scene.instance_mesh[-1]], np.uint32),
+        instance_material=np.asarray(first + [scene.instance_material[-1]], np.uint32),
+        object_to_world=m.astype(np.float32), world_to_object=np.linalg.inv(m).astype(np.float32), instance_names=[])
+    st = {"photons": 64, "bounces": 1, "gather_radius": 0.1}
+    g, o = Renderer.from_scene(scene, st), OracleRenderer(scene, st)
+    rays = _rays(20000, rng, 0.0, 1.0)
+    gi, gp, gt, _, _ = g.trace_rays(*rays)
+    oi, op, ot, _, _ = o.trace_rays(*rays)
+    g.close()
+    o.close()
+    assert len(np.unique(oi)) > instances // 2
+    assert np.mean(gi == oi) >= 0.9995
+    hit = (gi == oi) & (gi >= 0)
+    np.testing.assert_allclose(gt[hit], ot[hit], rtol=1e-5, atol=1e-6)
